@@ -383,13 +383,50 @@ struct GroupArgs {
   const float* scale;  // [groups, scale_ld] or null (never skip)
   int scale_ld;
   int l2_prefetch_kb;  // weight k-blocks to request into the L2 before the grid dependency (any launch)
-  // Token-gathered groups (mixture-of-experts dispatch): group z multiplies activation rows
-  // [row_offsets[z], row_offsets[z + 1]) (device array, written by the upstream kernel) and writes the same rows
-  // of Y; blockIdx.z = z * t_tiles + token tile (in every grouped launch), and a CTA whose tile lies past a gathered
-  // group's rows leaves at once.
+  // Token-gathered groups (mixture-of-experts dispatch): group g multiplies activation rows
+  // [row_offsets[g], row_offsets[g + 1]) (device array of n_groups + 1, written by the upstream kernel) and writes the
+  // same rows of Y.  The token tiles of all groups form one list, group after group; blockIdx.x is the place in that
+  // list and blockIdx.z the weight tile, so that the token tiles of a weight tile run next to one another and it is
+  // fetched from HBM once.  The grid has room for the longest list that the rows can make (gathered_tiles); CTAs past
+  // its end leave at once.  (A grid of every group's possible tiles would be mostly CTAs that leave: 3 of 4 at a
+  // prefill of 8 experts, 4 of 5 at 128 experts with a tile fitted to their few rows.)
+  // Other grouped launches: blockIdx.z = g * t_tiles + token tile.
   const int* row_offsets;
   int t_tiles;
+  int n_groups;  // gathered groups only
 };
+
+// Most token tiles that `rows` rows in `groups` groups of at most max_rows rows can make
+inline long long gathered_tiles(long long rows, int groups, int max_rows, int tn) {
+  const long long by_rows = rows / tn + groups, by_group = (long long)groups * ((max_rows + tn - 1) / tn);
+  return by_rows < by_group ? by_rows : by_group;
+}
+
+// Group and token tile at place `z` of the list of token tiles (tile = -1: past its end).  Every warp finds it for
+// itself, 32 groups at a time.
+__device__ __forceinline__ void gathered_tile(const int* off, int n_groups, int tn, int z, int& group, int& tile) {
+  const int lane = threadIdx.x & 31;
+  group = 0;
+  tile = -1;
+  for (int base = 0; base < n_groups; base += 32) {
+    const int g = base + lane;
+    const int mine = g < n_groups ? (off[g + 1] - off[g] + tn - 1) / tn : 0;
+    int upto = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += v;
+    }
+    const unsigned past = __ballot_sync(0xffffffffu, upto > z);
+    if (past) {
+      const int l = __ffs(past) - 1;
+      group = base + l;
+      tile = z - __shfl_sync(0xffffffffu, upto - mine, l);
+      return;
+    }
+    z -= __shfl_sync(0xffffffffu, upto, 31);
+  }
+}
 
 // 16 accumulator columns of this warp's TMEM lanes
 __device__ __forceinline__ void tmem_ld16_now(uint32_t taddr, uint32_t* r) {
@@ -425,16 +462,19 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
                  const QwArgs qw, const GroupArgs gr, const RopeArgs ro, const NormArgs nm) {
   constexpr bool MMQ = QT != QT_BF16;
   const bool gathered = gr.enabled && gr.row_offsets != nullptr;
-  const int zg = gr.enabled ? (int)blockIdx.z / gr.t_tiles : 0;
+  int zg = gr.enabled ? (int)blockIdx.z / gr.t_tiles : 0;
+  int tile_n = blockIdx.x, tile_t = gr.enabled ? (int)blockIdx.z % gr.t_tiles : (int)blockIdx.z;
   int g_row0 = 0;  // first activation / output row of this group (gathered groups)
   if (gathered) {
     pdl_wait();  // the row lists come from the upstream kernel
-    g_row0 = gr.row_offsets[zg];
-    T = gr.row_offsets[zg + 1] - g_row0;  // this group's own row count
-    if (((int)blockIdx.z % gr.t_tiles) * TN >= T) {
+    gathered_tile(gr.row_offsets, gr.n_groups, TN, blockIdx.x, zg, tile_t);
+    if (tile_t < 0) {
       pdl_launch_dependents();
       return;
     }
+    tile_n = blockIdx.z;
+    g_row0 = gr.row_offsets[zg];
+    T = gr.row_offsets[zg + 1] - g_row0;  // this group's own row count
   }
   if (gr.enabled && !gathered && gr.scale != nullptr) {
     // the routing weights come from the upstream kernel
@@ -479,7 +519,6 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
   // Plain launches with several token tiles walk the tile grid token-major: consecutive CTAs (one wave holds 148 of
   // them) share a weight tile and differ in the token tile, so a wave touches few weight tiles and all activation
   // tiles, both of which then stay in the L2, instead of every weight tile of the matrix in every wave.
-  int tile_n = blockIdx.x, tile_t = blockIdx.z;
   if (!gr.enabled && gridDim.z > 1 && gridDim.y == 1) {
     const int lin = blockIdx.z * gridDim.x + blockIdx.x;
     tile_n = lin / (int)gridDim.z;
@@ -487,7 +526,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
   }
   const int n0 = tile_n * GEMM_BM;
   const int split = blockIdx.y;
-  const int t0 = (gr.enabled ? (int)blockIdx.z % gr.t_tiles : tile_t) * TN;
+  const int t0 = tile_t * TN;
   const int w_row0 = n0 + zg * gr.w_rows;  // first weight row of this tile in the (stacked) matrix
   const int x_row0 = gathered ? g_row0 + t0 : t0 + zg * gr.x_rows;
   const int kb_total = (K + GEMM_BK - 1) / GEMM_BK;
@@ -1042,8 +1081,8 @@ inline GemmPlan gemm_plan(int T, int N, int K, int splits_hint, int sm_count, in
   if (T > 256 && sm_count > 0) {
     // Prefill-sized calls run one CTA per SM in waves; a nearly empty last wave costs a whole tile time.
     // 128-token tiles take half as long as 256-token ones, so compare the wave counts in half-tile units.
-    const long long w256 = ((long long)p.n_tiles * ((T + 255) / 256) + sm_count - 1) / sm_count * 2;
-    const long long w128 = ((long long)p.n_tiles * ((T + 127) / 128) + sm_count - 1) / sm_count;
+    const long long w256 = ((long long)p.n_tiles * groups * ((T + 255) / 256) + sm_count - 1) / sm_count * 2;
+    const long long w128 = ((long long)p.n_tiles * groups * ((T + 127) / 128) + sm_count - 1) / sm_count;
     if (g_oxb_gemm_prefill_tn == 128 || (g_oxb_gemm_prefill_tn == 0 && w128 < w256)) p.tn = 128;
   }
   p.t_tiles = (T + p.tn - 1) / p.tn;
@@ -1066,7 +1105,7 @@ inline GemmPlan gemm_plan(int T, int N, int K, int splits_hint, int sm_count, in
     long long best_cost = -1;
     splits = 1;
     const int s_max = p.tn <= 64 ? 16 : 4;  // wide tiles have large partials: a deep split costs more than it streams
-    for (int s = 1; s <= s_max && s <= max_by_k && (long long)tiles * s <= capacity && (s == 1 || tiles < sm_count); ++s) {
+    for (int s = 1; s <= s_max && s <= max_by_k && (long long)tiles * s <= capacity && (s == 1 || tiles * groups < sm_count); ++s) {
       const int per_cta = (kb_total + s - 1) / s;
       long long cost;
       if (packed) {
@@ -1078,7 +1117,7 @@ inline GemmPlan gemm_plan(int T, int N, int K, int splits_hint, int sm_count, in
         const int waves = (int)((ctas + (s > 1 ? slots : sm_count) - 1) / (s > 1 ? slots : sm_count));
         cost = (long long)waves * (per_cta + 12) + (s > 1 ? 2 + s / 4 + epi : 0);
       } else {
-        const int ctas_on_busiest = (tiles * s + sm_count - 1) / sm_count;
+        const int ctas_on_busiest = (tiles * groups * s + sm_count - 1) / sm_count;
         cost = (long long)ctas_on_busiest * (per_cta + 3) + (s > 1 ? 2 + s / 4 + epi : 0);
       }
       if (best_cost < 0 || cost < best_cost) {
@@ -1131,7 +1170,7 @@ template <int TN, int QT = QT_BF16>
 int gemm_launch(const CUtensorMap& tmW, const CUtensorMap& tmX, __nv_bfloat16* Y, const float* bias, int N, int T, int K,
                 int ldY, const GemmPlan& p, float* ws, int* counters, int epi_mode, const ArArgs& ar,
                 cudaStream_t stream, const QwArgs& qw = QwArgs{nullptr, 0, nullptr, 0},
-                const GroupArgs& gr = GroupArgs{0, 0, 0, 0, nullptr, 0, 0, nullptr, 1}, int groups = 1,
+                const GroupArgs& gr = GroupArgs{0, 0, 0, 0, nullptr, 0, 0, nullptr, 1, 0}, int groups = 1,
                 const RopeArgs& ro = RopeArgs{nullptr, nullptr, nullptr, 0, 0, 0, 0, 0, 0, 0, nullptr, nullptr},
                 const NormArgs& nm = NormArgs{nullptr, 0.f, 0.f, nullptr, nullptr}) {
   using Cfg = GemmTile<TN>;
@@ -1160,6 +1199,7 @@ int gemm_launch(const CUtensorMap& tmW, const CUtensorMap& tmX, __nv_bfloat16* Y
     if (splits > mc) splits = mc;
   }
   dim3 grid(p.n_tiles, splits, gr.enabled ? groups * gr.t_tiles : p.t_tiles);
+  if (gr.row_offsets != nullptr) grid = dim3(p.t_tiles, splits, p.n_tiles);  // p.t_tiles: the list's length
   const dim3 block(QT == QT_BF16 ? GEMM_THREADS : GEMM_THREADS_MMQ);
   cudaError_t le;
   GroupArgs grl = gr;
@@ -1180,7 +1220,7 @@ int gemm_launch(const CUtensorMap& tmW, const CUtensorMap& tmX, __nv_bfloat16* Y
 template <int QT>
 int gemm_launch_mmq(const CUtensorMap& tmX, __nv_bfloat16* Y, const float* bias, int N, int T, int K, int ldY,
                     const GemmPlan& p, float* ws, int* counters, int epi_mode, const ArArgs& ar, cudaStream_t stream,
-                    const QwArgs& qw, const GroupArgs& gr = GroupArgs{0, 0, 0, 0, nullptr, 0, 0, nullptr, 1}, int groups = 1,
+                    const QwArgs& qw, const GroupArgs& gr = GroupArgs{0, 0, 0, 0, nullptr, 0, 0, nullptr, 1, 0}, int groups = 1,
                     const CUtensorMap* tmWq = nullptr) {
   // tmWq: byte map of the packed rows (needed by the staged Q4_K path); other formats never touch tmW
   const CUtensorMap& tmW = tmWq != nullptr ? *tmWq : tmX;
