@@ -21,10 +21,10 @@ namespace oxb {
 constexpr int GEMM_BM = 128;  // weight rows per tile (UMMA M)
 constexpr int GEMM_BK = 64;   // bf16 per k-block = one 128-byte swizzle row
 // Warp roles.  Warps 0-3: epilogue (TMEM lane quarter = warp % 4).  Warp 4: TMA.  Warp 5: MMA issuer (owns the TMEM
-// allocation).  Packed weights add warps 6-7 (idle: they complete the second warpgroup, so that register budgets can be
-// moved between whole warpgroups) and, from warp 8 on, the dequant producers.
+// allocation).  Packed weights add warp 6 (TMA of the packed super-blocks), warp 7 (idle: it completes the second warpgroup, so
+// that register budgets can be moved between whole warpgroups) and, from warp 8 on, the dequant producers.
 constexpr int GEMM_THREADS = 192;
-constexpr int GEMM_WARP_TMA = 4, GEMM_WARP_MMA = 5, GEMM_WARP_PRODUCER0 = 8;
+constexpr int GEMM_WARP_TMA = 4, GEMM_WARP_MMA = 5, GEMM_WARP_PACKED = 6, GEMM_WARP_PRODUCER0 = 8;
 #ifndef OXB_MMQ_GROUPS
 #define OXB_MMQ_GROUPS 4
 #endif
@@ -32,7 +32,7 @@ constexpr int MMQ_GROUPS = OXB_MMQ_GROUPS;  // producer groups of four warps (on
 constexpr int GEMM_THREADS_MMQ = 32 * GEMM_WARP_PRODUCER0 + 128 * MMQ_GROUPS;
 // Register budgets of the packed-weight kernel (setmaxnreg): registers per thread at launch, then per warpgroup role.
 // A CTA can only redistribute what it was launched with, so the budgets must add up to exactly that.
-constexpr int MMQ_REGS_LAUNCH = 80, MMQ_REGS_EPILOGUE = 184, MMQ_REGS_CONTROL = 40, MMQ_REGS_PRODUCER = 64;
+constexpr int MMQ_REGS_LAUNCH = 80, MMQ_REGS_EPILOGUE = 152, MMQ_REGS_CONTROL = 40, MMQ_REGS_PRODUCER = 72;
 static_assert(128 * MMQ_REGS_EPILOGUE + 128 * MMQ_REGS_CONTROL + 128 * MMQ_GROUPS * MMQ_REGS_PRODUCER ==
                   GEMM_THREADS_MMQ * MMQ_REGS_LAUNCH,
               "warpgroup register budgets must add up to the launch allocation");
@@ -99,20 +99,24 @@ struct MmqStaged {
 template <int TN, int QT>
 struct GemmStages {
   static constexpr bool A_IN_TMEM = QT != QT_BF16;
-  static constexpr int STAGE_BYTES = A_IN_TMEM ? GemmTile<TN>::B_BYTES : GemmTile<TN>::STAGE_BYTES;
+  // k-blocks per stage.  Packed weights: two.  The control warps' instructions are what a k-block costs there: a wait, a vote, a
+  // fence, a commit and the addresses in between took the MMA warp 450 cycles next to the decoders, for 64 (16 tokens to a tile) to
+  // 256 (128 tokens) of tensor-core time; per pair of k-blocks they are paid once (Q4_K, 28672 x 4096, 32 tokens: 52 us before, 46 now).
+  static constexpr int KPS = A_IN_TMEM ? 2 : 1;
+  static constexpr int STAGE_BYTES = A_IN_TMEM ? KPS * GemmTile<TN>::B_BYTES : GemmTile<TN>::STAGE_BYTES;
   static constexpr int B_OFFSET = A_IN_TMEM ? 0 : GemmTile<TN>::A_BYTES;  // activation tile inside a stage
   static constexpr int TMEM_A_COLS = GEMM_BK / 2;                         // 32-bit columns of one decoded k-block
   // TMEM: accumulator first, then the A ring; the packed-weight kernel takes all 512 columns (it is alone on its SM).
   // Ring depth: bf16 weights use GemmTile's (the weight stream itself fills the ring).  For packed weights no unit of
   // the pipeline is saturated at decode sizes (decoders, TMA and MMA warps each wait a third of the time on the
   // others): what bounds the k-block rate is the number of k-blocks in flight, so the ring is as deep as tensor
-  // memory and shared memory allow, up to 12.
+  // memory and shared memory allow, up to 12 k-blocks.
   static constexpr int TMEM_COLS = A_IN_TMEM ? 512 : GemmTile<TN>::TMEM_COLS;
-  static constexpr int FIT_TMEM = (512 - GemmTile<TN>::ACC_COLS) / TMEM_A_COLS;
+  static constexpr int FIT_TMEM = (512 - GemmTile<TN>::ACC_COLS) / (KPS * TMEM_A_COLS);
   static constexpr int RING_BYTES = QT == QT_BF16 ? 0 : MmqRing<TN, QT>::value * MmqStage<QT>::BYTES;
   static constexpr int FIT_SMEM = (224 * 1024 - 1024 - 512 - 1024 - RING_BYTES) / (STAGE_BYTES > 0 ? STAGE_BYTES : 1);
   static constexpr int FIT = FIT_TMEM < FIT_SMEM ? FIT_TMEM : FIT_SMEM;
-  static constexpr int value = QT == QT_BF16 ? GemmTile<TN>::STAGES : (FIT > 12 ? 12 : FIT);
+  static constexpr int value = QT == QT_BF16 ? GemmTile<TN>::STAGES : (FIT > 6 ? 6 : FIT);
 };
 template <int TN, int QT>
 constexpr int gemm_smem_bytes() {
@@ -505,9 +509,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accum + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* ticket = const_cast<int*>(abort_flag) + 1;
-  // a producer group may run at most STAGES k-blocks ahead of the slowest one; with more groups than stages it could
-  // be two uses of a stage ahead, which the one-bit phase of the stage's barrier cannot tell apart
-  static_assert(!MMQ || STAGES >= MMQ_GROUPS, "the stage ring must be at least as deep as the number of producer groups");
+  // A producer group writes every second stage, so it may be two uses of a stage ahead of the last one that it waited for; that wait
+  // was for the stage two before, which is at least as far along as the use in question when there are two stages or more, so the
+  // one-bit phase of the barrier is unambiguous.
+  constexpr int KPS = St::KPS;
+  static_assert(!MMQ || (STAGES >= 2 && MMQ_GROUPS == 2 * KPS), "see above");
   static_assert(STAGES * STAGE_BYTES + PRING * MmqStage<QT>::BYTES >= TN * GEMM_BM * 6,
                 "the epilogue stages fp32 partials and a bf16 tile in the ring memory");
   static_assert(STAGES <= 12 && PRING <= 8, "barrier block layout");
@@ -533,12 +539,13 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
   const int kb_begin = (int)((long long)split * kb_total / splits);
   const int kb_end = (int)((long long)(split + 1) * kb_total / splits);
   const int nkb = kb_end - kb_begin;
+  const int nst = (nkb + KPS - 1) / KPS;  // uses of the stage ring
   // launched as clusters of `splits` CTAs along y: split-K reduces through distributed shared memory
   const bool csplit = splits > 1 && cluster_nctarank() == (uint32_t)splits;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < STAGES; ++i) {
-      mbar_init(&full[i], MMQ ? 1 + 4 : 1);  // TMA expect_tx arrival (+ one per producer warp of a group)
+      mbar_init(&full[i], MMQ ? 1 + 4 * KPS : 1);  // TMA expect_tx arrival (+ one per producer warp of a stage's groups)
       mbar_init(&empty[i], 1);
     }
     mbar_init(accum, 1);
@@ -581,7 +588,15 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     const bool leader = elect_one();
     const uint64_t pol_w = l2_policy_evict_first();  // weights are read once per step
     const uint64_t pol_x = l2_policy_evict_last();   // activations are re-read by every CTA
-    const int npre = nkb < STAGES ? nkb : STAGES;
+    const int npre = nst < STAGES ? nst : STAGES;
+    auto stage_kbs = [&](int i) { return KPS == 1 ? 1 : min(KPS, nkb - i * KPS); };  // k-blocks of the ring's i-th use
+    auto load_x = [&](int i, int st) {
+      uint8_t* sB = smem + st * STAGE_BYTES + St::B_OFFSET;
+#pragma unroll
+      for (int h = 0; h < KPS; ++h)
+        if (h == 0 || i * KPS + h < nkb)
+          tma_load_2d_hint(sB + h * Cfg::B_BYTES, &tmX, &full[st], (kb_begin + i * KPS + h) * GEMM_BK, x_row0, pol_x);
+    };
     if (leader) {
       tma_prefetch_desc(&tmW);
       tma_prefetch_desc(&tmX);
@@ -590,7 +605,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
       for (int i = 0; i < npre; ++i) {
         uint8_t* sA = smem + i * STAGE_BYTES;
         if constexpr (MMQ) {
-          mbar_expect_tx(&full[i], Cfg::B_BYTES);
+          mbar_expect_tx(&full[i], stage_kbs(i) * Cfg::B_BYTES);
         } else {
           mbar_expect_tx(&full[i], Cfg::STAGE_BYTES);
           tma_load_2d_hint(sA, &tmW, &full[i], (kb_begin + i) * GEMM_BK, w_row0, pol_w);
@@ -604,27 +619,21 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
       }
     }
     pdl_wait();  // activations come from the upstream kernel
-    if (leader) {
-      for (int i = 0; i < npre; ++i) {
-        uint8_t* sB = smem + i * STAGE_BYTES + St::B_OFFSET;
-        tma_load_2d_hint(sB, &tmX, &full[i], (kb_begin + i) * GEMM_BK, x_row0, pol_x);
-      }
-    }
-    int st = npre == STAGES ? 0 : npre;  // stage of k-block npre
+    if (leader)
+      for (int i = 0; i < npre; ++i) load_x(i, i);
+    int st = npre == STAGES ? 0 : npre;  // stage of the ring's use npre
     uint32_t ph = 0;                     // parity of the completion of empty[st] that frees it for its next use
-    for (int i = npre; i < nkb; ++i) {
+    for (int i = npre; i < nst; ++i) {
       const bool ok = OXB_TR_WAIT(tr_w0, mbar_wait_bounded(&empty[st], ph, abort_flag, OXB_TIMEOUT_TMA_EMPTY, blockIdx.x));
       if (!__all_sync(0xffffffffu, ok)) break;
       if (leader) {
-        uint8_t* sA = smem + st * STAGE_BYTES;
-        uint8_t* sB = sA + St::B_OFFSET;
         if constexpr (MMQ) {
-          mbar_expect_tx(&full[st], Cfg::B_BYTES);
+          mbar_expect_tx(&full[st], stage_kbs(i) * Cfg::B_BYTES);
         } else {
           mbar_expect_tx(&full[st], Cfg::STAGE_BYTES);
-          tma_load_2d_hint(sA, &tmW, &full[st], (kb_begin + i) * GEMM_BK, w_row0, pol_w);
+          tma_load_2d_hint(smem + st * STAGE_BYTES, &tmW, &full[st], (kb_begin + i) * GEMM_BK, w_row0, pol_w);
         }
-        tma_load_2d_hint(sB, &tmX, &full[st], (kb_begin + i) * GEMM_BK, x_row0, pol_x);
+        load_x(i, st);
       }
       if (++st == STAGES) {
         st = 0;
@@ -640,23 +649,31 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     const uint32_t smem_base = smem_u32(smem);
     int st = 0;
     uint32_t ph = 0;
-    for (int i = 0; i < nkb; ++i) {
+    for (int i = 0; i < nst; ++i) {
       const bool ok = OXB_TR_WAIT(tr_w0, mbar_wait_bounded(&full[st], ph, abort_flag, OXB_TIMEOUT_TMA_FULL, blockIdx.x));
       if (!__all_sync(0xffffffffu, ok)) break;
       tc_fence_after();
       if (leader) {
         const uint32_t a_addr = smem_base + st * STAGE_BYTES;
-        const uint64_t adesc = umma_desc_k_sw128(a_addr);
-        const uint64_t bdesc = umma_desc_k_sw128(a_addr + St::B_OFFSET);
         {
           OXB_TR_BEGIN
+          if constexpr (MMQ) {
+            const uint32_t ta = tmem_base + Cfg::ACC_COLS + st * (KPS * St::TMEM_A_COLS);
+            const uint32_t blo = umma_desc_lo(a_addr + St::B_OFFSET);
 #pragma unroll
-          for (int k = 0; k < GEMM_BK / 16; ++k) {
-            // advance 16 bf16 = 32 bytes inside the swizzle row: +2 in the (addr >> 4) field; in TMEM 16 bf16 = 8 columns
-            if constexpr (MMQ)
-              umma_bf16_ts(tmem_base, tmem_base + Cfg::ACC_COLS + st * St::TMEM_A_COLS + 8 * k, bdesc + 2 * k, idesc,
-                           (i > 0 || k > 0) ? 1u : 0u);
-            else
+            for (int h = 0; h < KPS; ++h) {
+              if (h > 0 && i * KPS + h >= nkb) break;
+#pragma unroll
+              for (int k = 0; k < GEMM_BK / 16; ++k)  // 16 bf16: 8 columns in TMEM
+                umma_bf16_ts_if(true, tmem_base, ta + h * St::TMEM_A_COLS + 8 * k, blo + h * (Cfg::B_BYTES >> 4) + 2 * k,
+                                UMMA_DESC_HI_SW128, idesc, h > 0 || k > 0 || i > 0);
+            }
+          } else {
+            const uint64_t adesc = umma_desc_k_sw128(a_addr);
+            const uint64_t bdesc = umma_desc_k_sw128(a_addr + St::B_OFFSET);
+#pragma unroll
+            for (int k = 0; k < GEMM_BK / 16; ++k)
+              // advance 16 bf16 = 32 bytes inside the swizzle row: +2 in the (addr >> 4) field
               umma_bf16(tmem_base, adesc + 2 * k, bdesc + 2 * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
           }
           OXB_TR_END(tr_w1)
@@ -683,6 +700,33 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     }
     __syncwarp();
     asm volatile("bar.arrive 3, 160;" ::: "memory");
+  } else if (warp == GEMM_WARP_PACKED) {
+    // ---------------- TMA producer of the packed super-blocks (tmW maps the packed rows as bytes): PRING boxes are in
+    // flight or being decoded; a box is refilled as soon as every decoding warp has let go of it.  Weights are static, so
+    // none of this waits for the upstream kernel.  (A thread of the first decoding group used to do this: its group then came
+    // last with every super-block, and as the MMAs take k-blocks in order, everything waited for it.)
+    if constexpr (STAGED) if (qw.staged) {
+      constexpr int SB = MmqStage<QT>::SB, PBYTES = MmqStage<QT>::BYTES;
+      const bool leader = elect_one();
+      const int sb_begin = kb_begin >> 2, sb_end = (kb_end + 3) >> 2;  // super-blocks touched by [kb_begin, kb_end)
+      if (leader) tma_prefetch_desc(&tmW);
+      int b = 0;
+      uint32_t ph = 1;  // parity of the use of box b before this one
+      for (int sb = sb_begin; sb < sb_end; ++sb) {
+        if (sb - sb_begin >= PRING) {
+          const bool ok = mbar_wait_bounded(&packed_empty[b], ph, abort_flag, OXB_TIMEOUT_TMA_EMPTY, blockIdx.x);
+          if (!__all_sync(0xffffffffu, ok)) break;
+        }
+        if (leader) {
+          mbar_expect_tx(&packed_full[b], PBYTES);
+          tma_load_2d(packed_buf + b * PBYTES, &tmW, &packed_full[b], ((sb * SB) & ~15) >> 2, w_row0);
+        }
+        if (++b == PRING) {
+          b = 0;
+          ph ^= 1;
+        }
+      }
+    }
   }
     __syncwarp();
     if (csplit) {
@@ -716,33 +760,41 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
       };
       // this thread's row of stage st in TMEM: lane = row (the warp's lane quarter is warp % 4), 32 columns per stage
       const uint32_t a_lane = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + Cfg::ACC_COLS;
-      auto wait_slot = [&](int i) -> bool {
-        const int st = i % STAGES;
-        const uint32_t ph = (i / STAGES) & 1;
+      // this group's place in a stage, and the stage of its next k-block with the parity of that use: the group's k-blocks
+      // (positions grp, grp + 4, ... of this CTA's) go to every second stage
+      const int half = grp & 1;
+      int st = grp >> 1;
+      uint32_t sph = 0;
+      auto wait_slot = [&]() -> bool {
         // warp-uniform verdict: the warp-level synchronisation below must be reached by all 32 lanes or none
-        const bool ok = OXB_TR_WAIT(tr_w0, __all_sync(0xffffffffu, mbar_wait_bounded(&empty[st], ph ^ 1, abort_flag,
+        const bool ok = OXB_TR_WAIT(tr_w0, __all_sync(0xffffffffu, mbar_wait_bounded(&empty[st], sph ^ 1, abort_flag,
                                                                                     OXB_TIMEOUT_TMA_EMPTY, blockIdx.x)));
         if (ok) tc_fence_after();  // the MMAs that read this slot are done: order this thread's TMEM stores after them
         return ok;
       };
-      auto signal_slot = [&](int i) {
+      auto signal_slot = [&]() {
         tmem_st_wait();     // this thread's stores have landed in TMEM
         tc_fence_before();  // ... and are ordered before the MMA thread's reads through the barrier
         __syncwarp();       // the warp's 32 rows are written: one arrival per warp instead of 32
-        if (lane == 0) mbar_arrive(&full[i % STAGES]);
+        if (lane == 0) mbar_arrive(&full[st]);
+        st += MMQ_GROUPS / KPS;
+        if (st >= STAGES) {
+          st -= STAGES;
+          sph ^= 1;
+        }
       };
-      auto publish = [&](int i, const uint32_t* v) -> bool {  // a k-block decoded into registers beforehand
-        if (!wait_slot(i)) return false;
-        const uint32_t dst = a_lane + (i % STAGES) * St::TMEM_A_COLS;
+      auto publish = [&](const uint32_t* v) -> bool {  // a k-block decoded into registers beforehand
+        if (!wait_slot()) return false;
+        const uint32_t dst = a_lane + (st * KPS + half) * St::TMEM_A_COLS;
 #pragma unroll
         for (int c = 0; c < 8; ++c) tmem_st4(dst + 4 * c, v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
-        signal_slot(i);
+        signal_slot();
         return true;
       };
       // staged form: wait for the ring slot first, then decode the row out of shared memory straight into it
-      auto publish_from = [&](int i, const uint8_t* srow, int kb) -> bool {
-        if (!wait_slot(i)) return false;
-        const uint32_t dst = a_lane + (i % STAGES) * St::TMEM_A_COLS;
+      auto publish_from = [&](const uint8_t* srow, int kb, int kq) -> bool {
+        if (!wait_slot()) return false;
+        const uint32_t dst = a_lane + (st * KPS + half) * St::TMEM_A_COLS;
         auto put = [&](int c, uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3) { tmem_st4(dst + 4 * c, w0, w1, w2, w3); };
         {
           OXB_TR_BEGIN
@@ -751,59 +803,43 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
           // the box holds there (zeros past the end of the matrix, the next expert's rows in a stacked one); the
           // epilogue never stores them.
           if constexpr (QT == QT_FP8B)  // scales are indexed by the absolute row and channel
-            dequant64_chunks<QT>(srow - (size_t)(kb & ~3) * GEMM_BK, kb * GEMM_BK, qw, n < N ? n : 0, put);
+            dequant64_chunks<QT>(srow - (size_t)(kb - kq) * GEMM_BK, kb * GEMM_BK, qw, n < N ? n : 0, put);
           else
-            dequant64_chunks<QT>(srow, (kb & 3) * GEMM_BK, qw, 0, put);
+            dequant64_chunks<QT>(srow, kq * GEMM_BK, qw, 0, put);
           OXB_TR_END(tr_w2)
         }
-        signal_slot(i);
+        signal_slot();
         return true;
       };
-      bool staged_done = false;
+      bool staged_done = false, alive = true;
       if constexpr (STAGED) if (qw.staged) {
         staged_done = true;
         constexpr int SB = MmqStage<QT>::SB, BOX = MmqStage<QT>::BOX, PBYTES = MmqStage<QT>::BYTES;
-        // Packed super-blocks arrive by TMA (tmW maps the packed rows as bytes): thread 192 keeps PRING - 1
-        // boxes in flight while one is decoded; all producers decode their own row out of shared memory and
-        // every warp releases a box when it is done with it.  Weights are static, so none of this waits for
-        // the upstream kernel.
+        static_assert(MMQ_GROUPS == 4, "a super-block holds one k-block for every group");
+        // Packed super-blocks arrive by TMA (warp GEMM_WARP_PACKED); all producers decode their own row out of shared
+        // memory and every warp releases a box when it is done with it.
+        // The instructions around a decode count: 16 warps walk every super-block, so with divisions, modulos and a loop
+        // over the other groups' k-blocks they came to more than the decoding itself (1530 issued per k-block, 660 of
+        // them the decoder's).  A group therefore knows its one k-block of every super-block, and ring positions are
+        // counters that wrap.
         const int sb_begin = kb_begin >> 2, sb_end = (kb_end + 3) >> 2;  // super-blocks touched by [kb_begin, kb_end)
-        const int nsb = sb_end - sb_begin;
-        auto sb_at = [&](int j) { return sb_begin + j; };  // j-th super-block of this CTA
-        auto issue = [&](int j) {  // j-th super-block in processing order -> box j % PRING
-          const int b = j % PRING;
-          mbar_expect_tx(&packed_full[b], PBYTES);
-          tma_load_2d(packed_buf + b * PBYTES, &tmW, &packed_full[b], ((sb_at(j) * SB) & ~15) >> 2, w_row0);
-        };
-        const bool issuer = r == 0 && grp == 0;
-        if (issuer) {
-          tma_prefetch_desc(&tmW);
-          for (int j = 0; j < PRING && j < nsb; ++j) issue(j);
-        }
-        bool alive = true;
-        for (int j = 0; j < nsb; ++j) {
-          const int b = j % PRING;
-          // the box of super-block j - 1 is refilled as soon as every warp has let go of it
-          if (issuer && alive && j >= 1 && j - 1 + PRING < nsb) {
-            if (OXB_TR_WAIT(tr_w1, mbar_wait_bounded(&packed_empty[(j - 1) % PRING], ((j - 1) / PRING) & 1, abort_flag,
-                                                     OXB_TIMEOUT_TMA_EMPTY, blockIdx.x)))
-              issue(j - 1 + PRING);
-          }
+        const int kq = (kb_begin + grp) & 3;  // this group's k-block inside a super-block: ring positions grp, grp + 4, ...
+        const uint8_t* const my_row = packed_buf + r * BOX;
+        int b = 0;         // box of this super-block
+        uint32_t bph = 0;  // ... and the parity of its use
+        for (int sb = sb_begin; sb < sb_end; ++sb) {
           if (alive)
-            alive = OXB_TR_WAIT(tr_w1, __all_sync(0xffffffffu, mbar_wait_bounded(&packed_full[b], (j / PRING) & 1, abort_flag,
+            alive = OXB_TR_WAIT(tr_w1, __all_sync(0xffffffffu, mbar_wait_bounded(&packed_full[b], bph, abort_flag,
                                                                                  OXB_TIMEOUT_TMA_FULL, blockIdx.x)));
-          if (alive) {
-            const int sb = sb_at(j);
-            const uint8_t* srow = packed_buf + b * PBYTES + r * BOX + ((sb * SB) & 15);
-            const int kb0 = max(kb_begin, sb * 4), kb1 = min(kb_end, sb * 4 + 4);
-            for (int kb = kb0; kb < kb1 && alive; ++kb) {
-              const int seq = kb - kb_begin;  // the ring's sequence number
-              if (seq % MMQ_GROUPS != grp) continue;  // another group's k-block
-              alive = publish_from(seq, srow, kb);
-            }
-          }
-          __syncwarp();  // the warp's reads of the box are done (alive or not, so that the issuer never waits in vain)
+          const int kb = 4 * sb + kq;
+          if (alive && kb >= kb_begin && kb < kb_end)
+            alive = publish_from(my_row + b * PBYTES + ((sb * SB) & 15), kb, kq);
+          __syncwarp();  // the warp's reads of the box are done (alive or not, so that its refill never waits in vain)
           if (lane == 0) mbar_arrive(&packed_empty[b]);
+          if (++b == PRING) {
+            b = 0;
+            bph ^= 1;
+          }
         }
       }
       if (!staged_done) {
@@ -813,9 +849,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
           uint32_t v0[32];
           decode(kb_begin + i, v0);
           mask(kb_begin + i, v0);
-          if (!publish(i, v0)) break;
+          alive = publish(v0);
+          if (!alive) break;
         }
       }
+      // an odd number of k-blocks leaves half of the last stage unwritten (and unread): its group arrives all the same
+      if (alive && nkb % KPS != 0 && grp == nkb % MMQ_GROUPS && wait_slot()) signal_slot();
       if (r == 0) { OXB_TR_STORE(2 + grp) }
     }
     __syncwarp();

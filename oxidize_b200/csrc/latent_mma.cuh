@@ -44,17 +44,6 @@ struct LatentMmaArgs {
   float scale_log2;
 };
 
-// An MN-major operand (64 contiguous values per 128-byte row, rows = the K dimension) with the 128-byte swizzle: 64-value
-// chunks lie the descriptor's leading offset apart, groups of 8 rows its stride offset (1024 bytes).
-constexpr uint32_t UMMA_A_MN_MAJOR = 1u << 15, UMMA_B_MN_MAJOR = 1u << 16;  // instruction descriptor bits
-
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
-      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
-      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-      : "memory");
-}
 // Reduce v[j] (j < 16) over the 32 lanes; lane L returns the result of j = L % 16.  v is used up.
 template <class Op>
 __device__ __forceinline__ float butterfly_rows(float* v, int lane, Op op) {

@@ -98,18 +98,6 @@ struct LatentPrefillArgs {
   float scale_log2;
 };
 
-__device__ __forceinline__ void umma_bf16_ts_if(bool issue, uint32_t tmem_d, uint32_t tmem_a, uint32_t blo, uint32_t bhi,
-                                                uint32_t idesc, bool accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t.reg .b64 db;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "setp.ne.b32 q, %5, 0;\n\t"
-      "mov.b64 db, {%2, %6};\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "r"(blo), "r"(idesc), "r"((uint32_t)accumulate), "r"((uint32_t)issue), "r"(bhi)
-      : "memory");
-}
-
 // Host: chunks and shared memory for a head's sizes; 0 bytes when the kernel does not cover them.
 struct LatentPrefillPlan {
   int nope_ch, rot_ch, v_ch, smem;
