@@ -44,6 +44,7 @@ struct AttnArgs {
   float* ws_o;   // [B*nkv*max_mtiles*n_cta_splits, 16, hd]
   float* ws_ml;  // [.., 16, 2]
   int* counters; // [B*nkv*max_mtiles] zero-initialised tickets (CTA splits only)
+  int max_rows;  // > 0: sequences that feed this many rows or more are another kernel's
   unsigned long long* trace;  // optional: phase timestamps (globaltimer ns) of CTA (0,0,0), for latency analysis
 };
 
@@ -218,6 +219,10 @@ paged_attention_kernel(const AttnArgs a, int G /*q heads per kv head*/) {
   const int mtile = blockIdx.x / a.n_cta_splits, csplit = blockIdx.x % a.n_cta_splits;
   const int q0 = a.query_start[b], qlen = a.query_start[b + 1] - q0;
   const int seq_len = a.seq_lens[b];
+  if (a.max_rows > 0 && qlen >= a.max_rows) {
+    pdl_wait();
+    return;
+  }
   const int R = qlen * G;
   const int row_base = mtile * 16;
   const size_t task = ((size_t)b * a.nkv + kvh) * gridDim.x + blockIdx.x;

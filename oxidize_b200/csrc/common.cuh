@@ -357,6 +357,9 @@ extern unsigned long long* g_oxb_attn_trace;
 // 2-D row-major tensor [rows, cols] of `elem_bytes` elements, box [box_rows, box_cols], 128B swizzle
 int oxb_make_tmap_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t row_stride_bytes,
                      uint32_t box_rows, uint32_t box_cols, int elem_bytes);
+// 3-D bf16 tensor (innermost size first), 128B swizzle
+int oxb_make_tmap_3d(CUtensorMap* out, const void* base, const uint64_t (&sizes)[3], const uint64_t (&strides_bytes)[2],
+                     const uint32_t (&box_sizes)[3]);
 
 // Programmatic dependent launch: a kernel started with this helper may begin (block scheduling,
 // shared-memory / barrier / TMEM set-up, loads of *static* data such as weights) while the previous

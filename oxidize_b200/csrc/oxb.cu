@@ -117,6 +117,22 @@ int oxb_make_tmap_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_t
   return r == CUDA_SUCCESS ? 0 : (int)cudaErrorInvalidValue;
 }
 
+int oxb_make_tmap_3d(CUtensorMap* out, const void* base, const uint64_t (&sizes)[3], const uint64_t (&strides_bytes)[2],
+                     const uint32_t (&box_sizes)[3]) {
+  PFN_encodeTiled enc = oxb_get_encode_tiled();
+  if (enc == nullptr) return (int)cudaErrorNotSupported;
+  if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || (strides_bytes[0] & 15) != 0 || (strides_bytes[1] & 15) != 0)
+    return (int)cudaErrorInvalidValue;
+  cuuint64_t dims[3] = {sizes[0], sizes[1], sizes[2]};
+  cuuint64_t strides[2] = {strides_bytes[0], strides_bytes[1]};
+  cuuint32_t box[3] = {box_sizes[0], box_sizes[1], box_sizes[2]};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : (int)cudaErrorInvalidValue;
+}
+
 // Byte view of packed weight rows for the staged MMQ path: [rows, row_bytes] uint8, no swizzle.
 int oxb_make_tmap_bytes(CUtensorMap* out, const void* base, uint64_t rows, uint64_t row_bytes, uint32_t box_rows,
                         uint32_t box_bytes) {

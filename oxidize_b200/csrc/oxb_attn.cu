@@ -1,6 +1,7 @@
 // liboxb, paged attention entry points.
 #include "common.cuh"
 #include "attention.cuh"
+#include "attention_prefill.cuh"
 using namespace oxb;
 
 // ----------------------------------------------------------------------------- attention
@@ -39,7 +40,7 @@ OXB_API int oxb_paged_attention(const void* q, void* out, const void* kv_data, c
                                 int max_blocks, int nq, int nkv, int hd, int kv_mode, int max_query_len,
                                 int n_cta_splits, int window, float scale, float softcap, const float* sink, int ld_out,
                                 float out_scale, float* ws_o, float* ws_ml, int* counters, int num_blocks,
-                                const void* gate, int ld_gate, int gate_per_value, cudaStream_t stream) {
+                                const void* gate, int ld_gate, int gate_per_value, int max_rows, cudaStream_t stream) {
   if (B <= 0) return 0;
   if (nq % nkv != 0 || (gate != nullptr && gate_per_value && (ld_gate % 2 != 0 || (reinterpret_cast<uintptr_t>(gate) & 3) != 0)))
     return (int)cudaErrorInvalidValue;
@@ -70,6 +71,7 @@ OXB_API int oxb_paged_attention(const void* q, void* out, const void* kv_data, c
   a.ws_ml = ws_ml;
   a.counters = counters;
   a.num_blocks = num_blocks;
+  a.max_rows = max_rows;
   a.trace = g_oxb_attn_trace;
   if (hd == 128) return attn_launch<128>(a, B, G, stream);
   if (hd == 64) return attn_launch<64>(a, B, G, stream);
@@ -81,3 +83,96 @@ OXB_API int oxb_paged_attention(const void* q, void* out, const void* kv_data, c
   return (int)cudaErrorInvalidValue;
 }
 
+
+// ----------------------------------------------------------------------------- long portions
+template <int HD>
+static int prefill_convert(int mode, const void* kv_data, const float* kv_scales, const int* block_tables, const int* seq_lens,
+                           const int* query_start, int B, int max_blocks, int num_blocks, int nkv, int max_pages, int cap_pages,
+                           int window, int min_rows, __nv_bfloat16* pages, cudaStream_t stream) {
+  const uint8_t* src = reinterpret_cast<const uint8_t*>(kv_data);
+  const dim3 grid(max_pages, B), block(256);
+  auto go = [&](auto kernel) {
+    return oxb_launch(kernel, grid, block, 0, stream, src, kv_scales, query_start, seq_lens, block_tables, max_blocks, num_blocks, nkv,
+                      window, min_rows, cap_pages, pages);
+  };
+  const cudaError_t e = mode == 1 ? go(prefill_pages_kernel<HD, 1>) : mode == 2 ? go(prefill_pages_kernel<HD, 2>) : go(prefill_pages_kernel<HD, 3>);
+  if (e != cudaSuccess) return (int)e;
+  OXB_CHECK_LAUNCH();
+  return 0;
+}
+
+template <int HD>
+static int prefill_launch(const void* q, const void* pages, AttnPrefillArgs a, int T, int nq, int max_query_len, cudaStream_t stream) {
+  static bool configured[64] = {false};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) return (int)cudaErrorInvalidDevice;
+  if (!configured[dev]) {
+    const cudaError_t e =
+        cudaFuncSetAttribute(paged_prefill_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_prefill_smem<HD>());
+    if (e != cudaSuccess) return (int)e;
+    configured[dev] = true;
+  }
+  CUtensorMap tq, tkv;
+  const uint64_t qs[3] = {(uint64_t)HD, (uint64_t)nq, (uint64_t)T}, qb[2] = {(uint64_t)HD * 2, (uint64_t)nq * HD * 2};
+  const uint32_t box[3] = {64, (uint32_t)a.gp, (uint32_t)(AP_M / a.gp)};
+  int e = oxb_make_tmap_3d(&tq, q, qs, qb, box);
+  if (e) return e;
+  e = oxb_make_tmap_2d(&tkv, pages, (uint64_t)a.num_blocks * a.nkv * 2 * ATT_PAGE, HD, (uint64_t)HD * 2, ATT_PAGE, 64, 2);
+  if (e) return e;
+  const int tok_per_cta = 2 * AP_M / a.gp;
+  const dim3 grid((max_query_len + tok_per_cta - 1) / tok_per_cta, nq / a.gp, a.B);
+  const cudaError_t le = oxb_launch(paged_prefill_kernel<HD>, grid, dim3(AP_THREADS), (size_t)attn_prefill_smem<HD>(), stream, tq, tkv, a);
+  if (le != cudaSuccess) return (int)le;
+  OXB_CHECK_LAUNCH();
+  return 0;
+}
+
+// 1 when oxb_paged_prefill covers heads of this width and these counts
+OXB_API int oxb_paged_prefill_supported(int hd, int nq, int nkv) {
+  return (hd == 64 || hd == 128) && nkv > 0 && nq % nkv == 0 && nq <= 65535;
+}
+
+// Attention of the sequences that feed at least min_rows rows (the others are left alone), arguments as oxb_paged_attention.
+// kv_mode > 0: `pages` [cap_pages, nkv, 2, 16, hd] bf16 receives their pages decoded (max_pages: of the longest context).
+OXB_API int oxb_paged_prefill(const void* q, void* out, const void* kv_data, const float* kv_scales, const int* block_tables,
+                              const int* seq_lens, const int* query_start, int B, int T, int max_blocks, int nq, int nkv, int hd,
+                              int kv_mode, int max_query_len, int min_rows, int window, float scale, const float* sink, int ld_out,
+                              float out_scale, int num_blocks, const void* gate, int ld_gate, int gate_per_value, void* pages,
+                              int cap_pages, int max_pages, cudaStream_t stream) {
+  if (B <= 0 || T <= 0 || max_query_len <= 0) return 0;
+  if (!oxb_paged_prefill_supported(hd, nq, nkv) || B > 65535 || kv_mode < 0 || kv_mode > 3 || ld_out % 2 != 0 ||
+      (kv_mode > 0 && (pages == nullptr || cap_pages <= 0 || max_pages <= 0)) ||
+      (gate != nullptr && gate_per_value && (ld_gate % 2 != 0 || (reinterpret_cast<uintptr_t>(gate) & 3) != 0)))
+    return (int)cudaErrorInvalidValue;
+  __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(pages);
+  if (kv_mode > 0) {
+    const int e = hd == 128 ? prefill_convert<128>(kv_mode, kv_data, kv_scales, block_tables, seq_lens, query_start, B, max_blocks, num_blocks,
+                                                   nkv, max_pages, cap_pages, window, min_rows, dst, stream)
+                            : prefill_convert<64>(kv_mode, kv_data, kv_scales, block_tables, seq_lens, query_start, B, max_blocks, num_blocks,
+                                                  nkv, max_pages, cap_pages, window, min_rows, dst, stream);
+    if (e) return e;
+  }
+  AttnPrefillArgs a;
+  a.query_start = query_start;
+  a.seq_lens = seq_lens;
+  a.block_tables = kv_mode > 0 ? nullptr : block_tables;
+  a.sink = sink;
+  a.out = reinterpret_cast<__nv_bfloat16*>(out);
+  a.B = B;
+  a.max_blocks = max_blocks;
+  a.num_blocks = kv_mode > 0 ? cap_pages : num_blocks;
+  a.nkv = nkv;
+  a.G = nq / nkv;
+  a.gp = 1;
+  while (a.gp < AP_M && a.G % (2 * a.gp) == 0) a.gp *= 2;  // the largest power of two that divides the group
+  a.window = window;
+  a.min_rows = min_rows;
+  a.ld_out = ld_out;
+  a.out_scale = out_scale;
+  a.scale_log2 = scale * 1.4426950408889634f;
+  a.gate = HeadGate{gate, ld_gate, gate_per_value};
+  const void* src = kv_mode > 0 ? pages : kv_data;
+  return hd == 128 ? prefill_launch<128>(q, src, a, T, nq, max_query_len, stream)
+                   : prefill_launch<64>(q, src, a, T, nq, max_query_len, stream);
+}

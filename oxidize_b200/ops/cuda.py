@@ -123,7 +123,9 @@ def _declare(L) -> None:
                                       i32, i32, vp]
     L.oxb_argmax.argtypes = [vp, i32, i32, i32, i32, vp, vp, i32, vp]
     L.oxb_paged_attention.argtypes = [vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, f32, f32,
-                                      vp, i32, f32, vp, vp, vp, i32, vp, i32, i32, vp]
+                                      vp, i32, f32, vp, vp, vp, i32, vp, i32, i32, i32, vp]
+    L.oxb_paged_prefill.argtypes = [vp] * 7 + [i32] * 10 + [f32, vp, i32, f32, i32, vp, i32, i32, vp, i32, i32, vp]
+    L.oxb_paged_prefill_supported.argtypes = [i32] * 3
     L.oxb_sample.argtypes = [vp, i32, i32, i32, vp, vp, vp, vp, vp, i32, vp, vp]
     L.oxb_gemm_quant.argtypes =[vp, vp, i32, sz, vp, i32, vp, vp, i32, i32, i32, i32, i32, i32, vp, sz, vp, i32, vp]
     u64p, ull = ctypes.POINTER(ctypes.c_uint64), ctypes.c_ulonglong
@@ -508,6 +510,39 @@ def attn_splits(B: int, nkv: int, mtiles: int, max_seq_len: int, sms: int) -> in
     return max(1, min(want, cap, 16))
 
 
+# Sequences that feed at least PREFILL_ROWS rows in a step take the tcgen05 kernel: it runs 256 (token, head) rows of a key head to
+# a CTA, the other 16.  8 sequences over 1000 rows, 32 heads / 8: 48 rows 35 against 80 us, 16 rows 33 against 33.
+PREFILL_ROWS = 32
+PREFILL_MAX_PAGES = 1 << 14  # ... their pages, where they have to be converted to bf16 first, up to this many in a step
+
+
+def _long_portions(q, kv, layer, meta) -> bool:
+    """Whether the step has portions for the tcgen05 kernel: their sizes are known on the host and it covers their heads."""
+    lens = getattr(meta, "host_lens", None)
+    if not lens or len(lens) != meta.seq_lens.shape[0] or kv.page_size != 16 or q.dtype != torch.bfloat16:
+        return False
+    pages = [(c + 15) // 16 for n, c in lens if n >= PREFILL_ROWS]
+    if not pages or (kv.dtype_name != "bf16" and sum(pages) > PREFILL_MAX_PAGES):
+        return False
+    return bool(lib().oxb_paged_prefill_supported(q.shape[2], q.shape[1], kv.spec.heads(layer)))
+
+
+def _paged_prefill(q, kv, layer, meta, scale, window, sink, out, out_scale, gate, gate_per_value) -> None:
+    T, nq, hd = q.shape
+    nkv = kv.spec.heads(layer)
+    long = [(n, c) for n, c in meta.host_lens if n >= PREFILL_ROWS]
+    pages, cap = None, 0
+    if kv.dtype_name != "bf16":
+        cap = sum((c + 15) // 16 for _, c in long)
+        pages = torch.empty(cap, nkv, 2, 16, hd, dtype=torch.bfloat16, device=q.device)
+    _check(lib().oxb_paged_prefill(q.data_ptr(), out.data_ptr(), kv.data[layer].data_ptr(), _p(kv.scales[layer]),
+                                   meta.block_tables.data_ptr(), meta.seq_lens.data_ptr(), meta.query_start.data_ptr(),
+                                   meta.seq_lens.shape[0], T, meta.block_tables.stride(0), nq, nkv, hd, KV_MODE[kv.dtype_name],
+                                   max(n for n, _ in long), PREFILL_ROWS, window, scale, _p(sink), out.stride(0), out_scale,
+                                   kv.num_blocks, _p(gate), 0 if gate is None else gate.stride(0), int(gate_per_value), _p(pages), cap,
+                                   max((c + 15) // 16 for _, c in long), _stream()), "oxb_paged_prefill")
+
+
 def paged_attention(q, kv, layer, meta, scale, sliding_window=0, splits: Optional[int] = None, softcap: float = 0.0,
                     sink: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None, out_scale: float = 1.0,
                     gate: Optional[torch.Tensor] = None, gate_per_value: bool = False):
@@ -517,14 +552,22 @@ def paged_attention(q, kv, layer, meta, scale, sliding_window=0, splits: Optiona
     nkv = kv.spec.heads(layer)
     B = meta.seq_lens.shape[0]
     G = nq // nkv
-    mtiles = (max(1, meta.max_query_len) * G + 15) // 16
+    if out is None:
+        out = torch.empty_like(q)
+    query_len, short_below = max(1, meta.max_query_len), 0
+    if splits is None and softcap == 0.0 and _long_portions(q, kv, layer, meta):
+        short_below = PREFILL_ROWS
+        _paged_prefill(q, kv, layer, meta, scale, sliding_window, sink, out, out_scale, gate, gate_per_value)
+        short = [n for n, _ in meta.host_lens if n < PREFILL_ROWS]
+        if not short:
+            return out
+        query_len = max(1, max(short))
+    mtiles = (query_len * G + 15) // 16
     if splits is None:
         span = meta.max_seq_len or kv.page_size
         if sliding_window > 0:
-            span = min(span, sliding_window + max(1, meta.max_query_len))
+            span = min(span, sliding_window + query_len)
         splits = attn_splits(B, nkv, mtiles, span, sm_count(q.device))
-    if out is None:
-        out = torch.empty_like(q)
     ws_o = ws_ml = cnt = None
     if splits > 1 and B * nkv * mtiles > scratch(q.device).attn_counters.numel():
         splits = 1
@@ -535,9 +578,9 @@ def paged_attention(q, kv, layer, meta, scale, sliding_window=0, splits: Optiona
     _check(lib().oxb_paged_attention(q.data_ptr(), out.data_ptr(), kv.data[layer].data_ptr(), _p(kv.scales[layer]),
                                      meta.block_tables.data_ptr(), meta.seq_lens.data_ptr(), meta.query_start.data_ptr(),
                                      B, meta.block_tables.stride(0), nq, nkv, hd, KV_MODE[kv.dtype_name],
-                                     max(1, meta.max_query_len), splits, sliding_window, scale, float(softcap), _p(sink),
+                                     query_len, splits, sliding_window, scale, float(softcap), _p(sink),
                                      out.stride(0), out_scale, _p(ws_o), _p(ws_ml), _p(cnt), kv.num_blocks, _p(gate),
-                                     0 if gate is None else gate.stride(0), int(gate_per_value), _stream()),
+                                     0 if gate is None else gate.stride(0), int(gate_per_value), short_below, _stream()),
            "oxb_paged_attention")
     return out
 
