@@ -7,7 +7,7 @@
 // cp.async ring, and keep their own online-softmax state; partial (max, sum, O) results are
 // merged in shared memory, and across CTA splits by whichever split finishes last (atomic ticket;
 // split-KV with exact log-sum-exp merge, no second launch).  KV pages may be bf16, f16, or the symmetric per-32-channel q8 / q4
-// encodings, which are decoded to bf16 on the way into shared memory.
+// encodings, whose codes become bf16 numbers in the fragments.
 //
 // Covers what the reference does with flash_attn_decode(_splitk/_reduce)
 // (oxidize-core/kernels/gemv_f32.cu:2035-2228), its CPU prefill attention
@@ -80,72 +80,73 @@ __device__ __forceinline__ void mma_bf16_16816(float* d, const uint32_t* a, uint
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// How a warp holds pages, by kind: MODE 0 are bf16 or f16 pages, 2 and 3 q8 and q4.
+// bf16 / f16 pages land as 32 rows of HD 16-bit values with row stride HD*2+16 bytes (bank-conflict-free ldmatrix); q8 / q4
+// pages land raw, 32 rows of codes 16 bytes further apart than they are long (so that the words which the lanes of a tensor-core
+// fragment take from eight rows lie on different banks), then 32 rows of scales.
+template <int HD, int MODE>
+struct AttPage {
+  static constexpr int CODES = MODE == 0 ? HD * 2 : MODE == 2 ? HD : HD / 2;  // bytes of a row
+  static constexpr int ROWB = CODES + 16;
+  static constexpr int NG = HD / 32;  // scales of a row
+  static constexpr int STAGE = 32 * ROWB + (MODE == 0 ? 0 : 32 * NG * 4);
+  // Quantized pages are a quarter to a half as long, and what bounds their kernel is instructions: three CTAs per SM.
+  static constexpr int STAGES = MODE == 3 ? 4 : ATT_STAGES;
+  static constexpr int SMEM = ATT_WARPS * STAGES * STAGE;
+  static_assert(SMEM >= ATT_WARPS * 16 * (HD + 2) * 4, "the warps' partial results are merged in the pages' memory");
+};
+
 // Bring one (K, V) page pair of a kv head into a warp-private stage with cp.async (one warp).
-// bf16 / f16 pages land as 32 rows of HD 16-bit values with row stride HD*2+16 bytes (bank-
-// conflict-free ldmatrix); q8 / q4 pages land raw: 32 rows of codes, then 32 rows of scales.
-template <int HD>
+template <int HD, int MODE>
 __device__ __forceinline__ void load_page(uint8_t* stage, const AttnArgs& a, int blk, int kvh, int lane) {
-  constexpr int ROWB = HD * 2 + 16;
+  using P = AttPage<HD, MODE>;
   const size_t page_idx = ((size_t)blk * a.nkv + kvh) * 2;  // K page; V page follows
-  if (a.kv_mode <= 1) {
-    const uint8_t* src = reinterpret_cast<const uint8_t*>(a.kv_data) + page_idx * ATT_PAGE * HD * 2;
-    constexpr int CPR = HD * 2 / 16;  // 16-byte chunks per row
+  const uint8_t* src = reinterpret_cast<const uint8_t*>(a.kv_data) + page_idx * ATT_PAGE * P::CODES;
+  constexpr int CPR = P::CODES / 16;  // 16-byte chunks per row
 #pragma unroll
-    for (int c = lane; c < 32 * CPR; c += 32) {
-      const int row = c / CPR, col = c % CPR;
-      cp_async16(stage + row * ROWB + col * 16, src + (size_t)c * 16);
-    }
-  } else {
-    const int rowbytes = a.kv_mode == 2 ? HD : HD / 2;
-    const uint8_t* src = reinterpret_cast<const uint8_t*>(a.kv_data) + page_idx * ATT_PAGE * rowbytes;
-    const uint8_t* sc = reinterpret_cast<const uint8_t*>(a.kv_scales + page_idx * ATT_PAGE * (HD / 32));
-    const int ncode = 32 * rowbytes / 16;
-    for (int c = lane; c < ncode; c += 32) cp_async16(stage + c * 16, src + (size_t)c * 16);
-    constexpr int NSC = 32 * (HD / 32) * 4 / 16;
-    for (int c = lane; c < NSC; c += 32) cp_async16(stage + 32 * rowbytes + c * 16, sc + (size_t)c * 16);
+  for (int c = lane; c < 32 * CPR; c += 32) {
+    const int row = c / CPR, col = c % CPR;
+    cp_async16(stage + row * P::ROWB + col * 16, src + (size_t)c * 16);
+  }
+  if constexpr (MODE != 0) {
+    const uint8_t* sc = reinterpret_cast<const uint8_t*>(a.kv_scales + page_idx * ATT_PAGE * P::NG);
+    constexpr int NSC = 32 * P::NG * 4 / 16;
+    for (int c = lane; c < NSC; c += 32) cp_async16(stage + 32 * P::ROWB + c * 16, sc + (size_t)c * 16);
   }
 }
 
-// f16 pages: convert to bf16 in place.  q8 / q4 pages: decode codes * scale into `dec` (bf16,
-// padded rows).  One warp; the caller synchronises the warp before the tensor-core reads.
+// f16 pages: convert to bf16 in place.  One warp; the caller synchronises the warp before the tensor-core reads.
 template <int HD>
-__device__ __forceinline__ void decode_page(uint8_t* stage, uint8_t* dec, int kv_mode, int lane) {
+__device__ __forceinline__ void decode_page(uint8_t* stage, int lane) {
   constexpr int ROWB = HD * 2 + 16;
-  if (kv_mode == 1) {
-    for (int c = lane; c < 32 * HD / 2; c += 32) {
-      const int row = c / (HD / 2), col = (c % (HD / 2)) * 2;
-      uint32_t* p = reinterpret_cast<uint32_t*>(stage + row * ROWB + col * 2);
-      const float2 f = __half22float2(*reinterpret_cast<const __half2*>(p));
-      *p = pack_bf16x2(f.x, f.y);
-    }
-  } else {
-    const bool q8 = kv_mode == 2;
-    const int rowbytes = q8 ? HD : HD / 2;
-    const float* sc = reinterpret_cast<const float*>(stage + 32 * rowbytes);
-    for (int c = lane; c < 32 * HD / 8; c += 32) {  // 8 channels per step
-      const int row = c / (HD / 8), col = (c % (HD / 8)) * 8;
-      const float s = sc[row * (HD / 32) + (col >> 5)];
-      float v[8];
-      if (q8) {
-        const uint2 w = *reinterpret_cast<const uint2*>(stage + row * rowbytes + col);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          v[j] = ((float)((w.x >> (8 * j)) & 0xFF) - 127.f) * s;
-          v[4 + j] = ((float)((w.y >> (8 * j)) & 0xFF) - 127.f) * s;
-        }
-      } else {
-        const uint32_t w = *reinterpret_cast<const uint32_t*>(stage + row * rowbytes + (col >> 1));
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = ((float)((w >> (4 * j)) & 0xF) - 7.f) * s;
-      }
-      uint4 o;
-      o.x = pack_bf16x2(v[0], v[1]);
-      o.y = pack_bf16x2(v[2], v[3]);
-      o.z = pack_bf16x2(v[4], v[5]);
-      o.w = pack_bf16x2(v[6], v[7]);
-      *reinterpret_cast<uint4*>(dec + row * ROWB + col * 2) = o;
-    }
+  for (int c = lane; c < 32 * HD / 2; c += 32) {
+    const int row = c / (HD / 2), col = (c % (HD / 2)) * 2;
+    uint32_t* p = reinterpret_cast<uint32_t*>(stage + row * ROWB + col * 2);
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(p));
+    *p = pack_bf16x2(f.x, f.y);
   }
+}
+
+// Codes of quantized pages as bf16 pairs, exactly: a code below 128 in the mantissa of 128.0 (0x4300) is the bf16 number
+// 128 + code, and what is subtracted from it is exact too.  The scales stay out of it: they are applied in 32 bits to the sums over
+// their 32 channels (keys) or to the probabilities (values).
+__device__ __forceinline__ uint32_t att_sub2(uint32_t x, uint32_t y) {
+  const __nv_bfloat162 d = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&x), *reinterpret_cast<const __nv_bfloat162*>(&y));
+  return *reinterpret_cast<const uint32_t*>(&d);
+}
+// q4: nibbles 0 and 4 of w, less 7 (128 + code - 135)
+__device__ __forceinline__ uint32_t att_q4_pair(uint32_t w) { return att_sub2((w & 0x000F000Fu) | 0x43004300u, 0x43074307u); }
+// q8: bytes 0 and 2 of w, less 127.  The top bit of a code (`sign`: it, repeated over its half) decides between
+// 128 + low bits - 255 and 128 + low bits - 127.
+__device__ __forceinline__ uint32_t att_q8_pair(uint32_t w, uint32_t sign) {
+  return att_sub2((w & 0x007F007Fu) | 0x43004300u, 0x437F437Fu ^ (sign & 0x01810181u));
+}
+// PRMT whose selectors may ask for a byte's sign, repeated (top bit of a nibble)
+template <uint32_t SEL>
+__device__ __forceinline__ uint32_t att_prmt(uint32_t x, uint32_t y) {
+  uint32_t d;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(x), "r"(y), "n"(SEL));
+  return d;
 }
 
 // Factor of an output row by its head's gate, and of two neighbouring values by theirs (1 where there is none).
@@ -200,11 +201,17 @@ __device__ __forceinline__ void attn_merge_rows(const AttnArgs& a, int G, int b,
   }
 }
 
-template <int HD>
-__global__ void __launch_bounds__(ATT_WARPS * 32)
+// Quantized pages are read into the tensor-core fragments straight from their codes.  The order of the channels inside a sum
+// and that of the output columns are free, so a lane takes whole words of codes: of a key's 32 channels under one scale, lane t4 takes
+// 8t4 .. 8t4 + 7, and the queries' fragments are put in the same order; of a value row's, lane g takes 4g .. 4g + 3, one for each of four
+// column tiles.  The sums of a key's channel groups are scaled apart, as are the probabilities for the values' groups.
+// (Decoding pages to bf16 rows in shared memory first took 1150 instructions a page and 139 KB, one CTA per SM: at 4 x 25000 q4 rows of
+// 8 heads, 128 wide, 273 us, now 65, of which the copies would take 20; 32 x 640 q8 rows 63 and 25.)
+template <int HD, int MODE>
+__global__ void __launch_bounds__(ATT_WARPS * 32, MODE == 0 ? 1 : 3)
 paged_attention_kernel(const AttnArgs a, int G /*q heads per kv head*/) {
-  constexpr int ROWB = HD * 2 + 16;
-  constexpr int STAGE_BYTES = 32 * ROWB;
+  using Page = AttPage<HD, MODE>;
+  constexpr int ROWB = Page::ROWB, STAGE_BYTES = Page::STAGE, STAGES = Page::STAGES, NG = Page::NG;
   constexpr int KS = HD / 16;  // k-steps for QK^T
   constexpr int NT = HD / 8;   // n-tiles of the output
   extern __shared__ __align__(16) uint8_t att_smem[];
@@ -257,7 +264,7 @@ paged_attention_kernel(const AttnArgs a, int G /*q heads per kv head*/) {
   for (int nt = 0; nt < NT; ++nt) o[nt][0] = o[nt][1] = o[nt][2] = o[nt][3] = 0.f;
   float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
 
-  uint8_t* my_stage = att_smem + (size_t)warp * ATT_STAGES * STAGE_BYTES;
+  uint8_t* my_stage = att_smem + (size_t)warp * STAGES * STAGE_BYTES;
   const int* bt = a.block_tables + (size_t)b * a.max_blocks;
   // Page ids of this warp, fetched 32 at a time into registers (two batches held) so that the
   // block-table load never sits in front of a page load on the critical path.
@@ -282,21 +289,41 @@ paged_attention_kernel(const AttnArgs a, int G /*q heads per kv head*/) {
   ATT_STAMP(1);
   // Q fragments (A operand), straight from global memory
   uint32_t qf[KS][4];
+  if constexpr (MODE == 0) {
 #pragma unroll
-  for (int ks = 0; ks < KS; ++ks) {
+    for (int ks = 0; ks < KS; ++ks) {
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const __nv_bfloat16* qp = a.q + ((size_t)(q0 + qtok[i]) * a.nq + kvh * G + hg[i]) * HD + ks * 16 + 2 * t4;
-      qf[ks][i] = rvalid[i] ? *reinterpret_cast<const uint32_t*>(qp) : 0u;
-      qf[ks][i + 2] = rvalid[i] ? *reinterpret_cast<const uint32_t*>(qp + 8) : 0u;
+      for (int i = 0; i < 2; ++i) {
+        const __nv_bfloat16* qp = a.q + ((size_t)(q0 + qtok[i]) * a.nq + kvh * G + hg[i]) * HD + ks * 16 + 2 * t4;
+        qf[ks][i] = rvalid[i] ? *reinterpret_cast<const uint32_t*>(qp) : 0u;
+        qf[ks][i + 2] = rvalid[i] ? *reinterpret_cast<const uint32_t*>(qp + 8) : 0u;
+      }
+    }
+  } else {
+#pragma unroll
+    for (int gi = 0; gi < NG; ++gi) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const uint32_t* qp =
+            reinterpret_cast<const uint32_t*>(a.q + ((size_t)(q0 + qtok[i]) * a.nq + kvh * G + hg[i]) * HD + gi * 32 + 8 * t4);
+        uint32_t w[4];  // channels (0, 1) (2, 3) (4, 5) (6, 7) of this lane's eight
+#pragma unroll
+        for (int j = 0; j < 4; ++j) w[j] = rvalid[i] ? qp[j] : 0u;
+        constexpr int X = 0, Y = MODE == 3 ? 2 : 1, Z = MODE == 3 ? 1 : 2, W = 3;
+        // q4: (0, 4) (1, 5) | (2, 6) (3, 7), the nibbles that lie 16 bits apart; q8: (0, 2) (1, 3) | (4, 6) (5, 7)
+        qf[2 * gi][i] = att_prmt<0x5410>(w[X], w[Y]);
+        qf[2 * gi][i + 2] = att_prmt<0x7632>(w[X], w[Y]);
+        qf[2 * gi + 1][i] = att_prmt<0x5410>(w[Z], w[W]);
+        qf[2 * gi + 1][i + 2] = att_prmt<0x7632>(w[Z], w[W]);
+      }
     }
   }
 
   ATT_STAMP(2);
   // prologue: fill the ring
 #pragma unroll
-  for (int s = 0; s < ATT_STAGES - 1; ++s) {
-    if (s < my_pages) load_page<HD>(my_stage + s * STAGE_BYTES, a, page_id(s), kvh, lane);
+  for (int s = 0; s < STAGES - 1; ++s) {
+    if (s < my_pages) load_page<HD, MODE>(my_stage + s * STAGE_BYTES, a, page_id(s), kvh, lane);
     cp_async_commit();
   }
 
@@ -306,33 +333,59 @@ paged_attention_kernel(const AttnArgs a, int G /*q heads per kv head*/) {
       ids_a = ids_b;
       ids_b = (id_base + 32 + lane < my_pages) ? bt[page_lo + first + (id_base + 32 + lane) * stride] : 0;
     }
-    const int nxt = it + ATT_STAGES - 1;
-    if (nxt < my_pages) load_page<HD>(my_stage + (nxt % ATT_STAGES) * STAGE_BYTES, a, page_id(nxt), kvh, lane);
+    const int nxt = it + STAGES - 1;
+    if (nxt < my_pages) load_page<HD, MODE>(my_stage + (nxt % STAGES) * STAGE_BYTES, a, page_id(nxt), kvh, lane);
     cp_async_commit();
-    cp_async_wait<ATT_STAGES - 1>();
+    cp_async_wait<STAGES - 1>();
     __syncwarp();
     if (it == 0) ATT_STAMP(3);
-    uint8_t* st = my_stage + (it % ATT_STAGES) * STAGE_BYTES;
-    if (a.kv_mode != 0) {
-      uint8_t* dec = att_smem + (size_t)(ATT_WARPS * ATT_STAGES + warp) * STAGE_BYTES;
-      decode_page<HD>(st, dec, a.kv_mode, lane);
-      if (a.kv_mode >= 2) st = dec;
+    uint8_t* st = my_stage + (it % STAGES) * STAGE_BYTES;
+    if (MODE == 0 && a.kv_mode != 0) {
+      decode_page<HD>(st, lane);
       __syncwarp();
     }
-    const uint32_t k_base = smem_u32(st), v_base = k_base + 16 * ROWB;
     const int page = page_lo + first + it * stride;
 
     // S = Q K^T for 16 tokens: 2 n-tiles
     float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-    {
+    if constexpr (MODE == 0) {
       const int mi = lane >> 3, r = lane & 7;
-      const uint32_t addr0 = k_base + ((mi >> 1) * 8 + r) * ROWB + (mi & 1) * 16;
+      const uint32_t addr0 = smem_u32(st) + ((mi >> 1) * 8 + r) * ROWB + (mi & 1) * 16;
 #pragma unroll
       for (int ks = 0; ks < KS; ++ks) {
         uint32_t b0, b1, b2, b3;
         ldmatrix_x4(addr0 + ks * 32, b0, b1, b2, b3);
         mma_bf16_16816(s[0], qf[ks], b0, b1);
         mma_bf16_16816(s[1], qf[ks], b2, b3);
+      }
+    } else {
+      const float* sc = reinterpret_cast<const float*>(st + 32 * ROWB) + 2 * t4 * NG;  // scales of keys 2 t4, 2 t4 + 1 (+ 8)
+#pragma unroll
+      for (int gi = 0; gi < NG; ++gi) {
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+          const uint8_t* row = st + (nt * 8 + g) * ROWB;
+          uint32_t b[4];
+          if constexpr (MODE == 3) {
+            const uint32_t w = *reinterpret_cast<const uint32_t*>(row + gi * 16 + t4 * 4);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) b[j] = att_q4_pair(w >> (4 * j));
+          } else {
+            const uint2 w = *reinterpret_cast<const uint2*>(row + gi * 32 + t4 * 8);
+            b[0] = att_q8_pair(w.x, att_prmt<0xAA88>(w.x, 0u));
+            b[1] = att_q8_pair(w.x >> 8, att_prmt<0xBB99>(w.x, 0u));
+            b[2] = att_q8_pair(w.y, att_prmt<0xAA88>(w.y, 0u));
+            b[3] = att_q8_pair(w.y >> 8, att_prmt<0xBB99>(w.y, 0u));
+          }
+          float part[4] = {0.f, 0.f, 0.f, 0.f};
+          mma_bf16_16816(part, qf[2 * gi], b[0], b[1]);
+          mma_bf16_16816(part, qf[2 * gi + 1], b[2], b[3]);
+          const float k0 = sc[nt * 8 * NG + gi], k1 = sc[(nt * 8 + 1) * NG + gi];
+          s[nt][0] += part[0] * k0;
+          s[nt][1] += part[1] * k1;
+          s[nt][2] += part[2] * k0;
+          s[nt][3] += part[3] * k1;
+        }
       }
     }
     // scale, mask, online softmax (rows g and g+8; a quad holds one row's 16 scores)
@@ -379,20 +432,50 @@ paged_attention_kernel(const AttnArgs a, int G /*q heads per kv head*/) {
       }
     }
     // O += P V : P (16x16) as A fragment, V page as B via transposing ldmatrix
-    uint32_t pf[4];
-    pf[0] = pack_bf16x2(p[0][0], p[0][1]);
-    pf[1] = pack_bf16x2(p[0][2], p[0][3]);
-    pf[2] = pack_bf16x2(p[1][0], p[1][1]);
-    pf[3] = pack_bf16x2(p[1][2], p[1][3]);
-    {
+    if constexpr (MODE == 0) {
+      uint32_t pf[4];
+      pf[0] = pack_bf16x2(p[0][0], p[0][1]);
+      pf[1] = pack_bf16x2(p[0][2], p[0][3]);
+      pf[2] = pack_bf16x2(p[1][0], p[1][1]);
+      pf[3] = pack_bf16x2(p[1][2], p[1][3]);
       const int mi = lane >> 3, r = lane & 7;
-      const uint32_t addr0 = v_base + ((mi & 1) * 8 + r) * ROWB + (mi >> 1) * 16;
+      const uint32_t addr0 = smem_u32(st) + 16 * ROWB + ((mi & 1) * 8 + r) * ROWB + (mi >> 1) * 16;
 #pragma unroll
       for (int nt = 0; nt < NT; nt += 2) {
         uint32_t b0, b1, b2, b3;
         ldmatrix_x4_trans(addr0 + nt * 16, b0, b1, b2, b3);
         mma_bf16_16816(o[nt], pf, b0, b1);
         mma_bf16_16816(o[nt + 1], pf, b2, b3);
+      }
+    } else {
+      // this lane's tokens are 2 t4, 2 t4 + 1 and those 8 further; column n of tile 4 gi + j is channel 32 gi + 4 n + j
+      const float* sc = reinterpret_cast<const float*>(st + 32 * ROWB) + (16 + 2 * t4) * NG;
+      const uint8_t* row = st + (16 + 2 * t4) * ROWB;
+#pragma unroll
+      for (int gi = 0; gi < NG; ++gi) {
+        uint32_t pf[4], b[2][4];
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+          const float v0 = sc[nt * 8 * NG + gi], v1 = sc[(nt * 8 + 1) * NG + gi];
+          pf[2 * nt] = pack_bf16x2(p[nt][0] * v0, p[nt][1] * v1);
+          pf[2 * nt + 1] = pack_bf16x2(p[nt][2] * v0, p[nt][3] * v1);
+          const uint8_t* r0 = row + nt * 8 * ROWB;
+          if constexpr (MODE == 3) {
+            const uint32_t w = (uint32_t)*reinterpret_cast<const uint16_t*>(r0 + gi * 16 + 2 * g) |
+                               (uint32_t)*reinterpret_cast<const uint16_t*>(r0 + ROWB + gi * 16 + 2 * g) << 16;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) b[nt][j] = att_q4_pair(w >> (4 * j));
+          } else {
+            const uint32_t x = *reinterpret_cast<const uint32_t*>(r0 + gi * 32 + 4 * g);
+            const uint32_t y = *reinterpret_cast<const uint32_t*>(r0 + ROWB + gi * 32 + 4 * g);
+            b[nt][0] = att_q8_pair(att_prmt<0x5410>(x, y), att_prmt<0xCC88>(x, y));
+            b[nt][1] = att_q8_pair(att_prmt<0x6521>(x, y), att_prmt<0xDD99>(x, y));
+            b[nt][2] = att_q8_pair(att_prmt<0x7632>(x, y), att_prmt<0xEEAA>(x, y));
+            b[nt][3] = att_q8_pair(att_prmt<0x7733>(x, y), att_prmt<0xFFBB>(x, y));
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) mma_bf16_16816(o[4 * gi + j], pf, b[0][j], b[1][j]);
       }
     }
     __syncwarp();
@@ -412,8 +495,15 @@ paged_attention_kernel(const AttnArgs a, int G /*q heads per kv head*/) {
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       if (rvalid[i]) {
-        float2* dst = reinterpret_cast<float2*>(mo + ((size_t)warp * 16 + g + 8 * i) * HD + nt * 8 + 2 * t4);
-        *dst = make_float2(o[nt][2 * i], o[nt][2 * i + 1]);
+        float* row = mo + ((size_t)warp * 16 + g + 8 * i) * HD;
+        if constexpr (MODE == 0) {
+          *reinterpret_cast<float2*>(row + nt * 8 + 2 * t4) = make_float2(o[nt][2 * i], o[nt][2 * i + 1]);
+        } else if ((nt & 3) == 0) {  // four tiles hold eight neighbouring channels
+#pragma unroll
+          for (int e = 0; e < 2; ++e)
+            *reinterpret_cast<float4*>(row + 8 * nt + 8 * t4 + 4 * e) =
+                make_float4(o[nt][2 * i + e], o[nt + 1][2 * i + e], o[nt + 2][2 * i + e], o[nt + 3][2 * i + e]);
+        }
       }
     }
   }

@@ -14,15 +14,12 @@ OXB_API int oxb_attn_ws_floats(int B, int nkv, int max_mtiles, int n_cta_splits,
   return 0;
 }
 
-template <int HD>
+template <int HD, int MODE = 0>
 static int attn_launch(const AttnArgs& a, int B, int G, cudaStream_t stream) {
-  constexpr int STAGE = 32 * (HD * 2 + 16);
-  constexpr int SMEM_MAX = ATT_WARPS * (ATT_STAGES + (HD <= 128 ? 1 : 0)) * STAGE;
-  // quantized KV needs one extra decode buffer per warp
-  const int smem = ATT_WARPS * (ATT_STAGES + (a.kv_mode >= 2 ? 1 : 0)) * STAGE;
+  constexpr int smem = AttPage<HD, MODE>::SMEM;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(paged_attention_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX);
+    cudaError_t e = cudaFuncSetAttribute(paged_attention_kernel<HD, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
@@ -30,7 +27,7 @@ static int attn_launch(const AttnArgs& a, int B, int G, cudaStream_t stream) {
   // (The KV splits of a row tile stay independent CTAs and the last one to finish merges: inside a thread-block
   // cluster every CTA would wait for the slowest split.)
   if (a.n_cta_splits > 1 && (a.ws_o == nullptr || a.ws_ml == nullptr || a.counters == nullptr)) return (int)cudaErrorInvalidValue;
-  oxb_launch(paged_attention_kernel<HD>, grid, dim3(ATT_WARPS * 32), (size_t)smem, stream, a, G);
+  oxb_launch(paged_attention_kernel<HD, MODE>, grid, dim3(ATT_WARPS * 32), (size_t)smem, stream, a, G);
   OXB_CHECK_LAUNCH();
   return 0;
 }
@@ -73,6 +70,10 @@ OXB_API int oxb_paged_attention(const void* q, void* out, const void* kv_data, c
   a.num_blocks = num_blocks;
   a.max_rows = max_rows;
   a.trace = g_oxb_attn_trace;
+  if (kv_mode == 2 && hd == 128) return attn_launch<128, 2>(a, B, G, stream);
+  if (kv_mode == 2 && hd == 64) return attn_launch<64, 2>(a, B, G, stream);
+  if (kv_mode == 3 && hd == 128) return attn_launch<128, 3>(a, B, G, stream);
+  if (kv_mode == 3 && hd == 64) return attn_launch<64, 3>(a, B, G, stream);
   if (hd == 128) return attn_launch<128>(a, B, G, stream);
   if (hd == 64) return attn_launch<64>(a, B, G, stream);
   if (kv_mode != 0) return (int)cudaErrorInvalidValue;

@@ -499,12 +499,12 @@ def sm_count(device) -> int:
     return _SM_COUNT[idx]
 
 
-def attn_splits(B: int, nkv: int, mtiles: int, max_seq_len: int, sms: int) -> int:
-    """CTA-level KV splits: as many as keep the grid within ONE wave of two CTAs per SM (a partly
-    filled second wave doubles the kernel's time) while each warp of each split still sees a few
+def attn_splits(B: int, nkv: int, mtiles: int, max_seq_len: int, sms: int, per_sm: int = 2) -> int:
+    """CTA-level KV splits: as many as keep the grid within ONE wave of ``per_sm`` CTAs per SM (two, or three over
+    quantized pages; a partly filled second wave doubles the kernel's time) while each warp of each split still sees a few
     pages."""
     base = max(1, B * nkv * mtiles)
-    want = max(1, (2 * sms) // base)
+    want = max(1, (per_sm * sms) // base)
     pages = max(1, (max_seq_len + 15) // 16)
     cap = max(1, pages // 8)  # >= 2 pages per warp per split
     return max(1, min(want, cap, 16))
@@ -567,7 +567,7 @@ def paged_attention(q, kv, layer, meta, scale, sliding_window=0, splits: Optiona
         span = meta.max_seq_len or kv.page_size
         if sliding_window > 0:
             span = min(span, sliding_window + query_len)
-        splits = attn_splits(B, nkv, mtiles, span, sm_count(q.device))
+        splits = attn_splits(B, nkv, mtiles, span, sm_count(q.device), 3 if kv.dtype_name in ("q8", "q4") else 2)
     ws_o = ws_ml = cnt = None
     if splits > 1 and B * nkv * mtiles > scratch(q.device).attn_counters.numel():
         splits = 1
