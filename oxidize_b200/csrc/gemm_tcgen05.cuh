@@ -81,10 +81,13 @@ struct MmqStage {
 };
 // bytes fetched per row for a packed format (host side)
 inline int mmq_box_bytes(int qtype) { return qtype == QT_Q6_K ? 240 : (qtype == QT_Q8_0 || qtype == QT_FP8B) ? 272 : 144; }
-// boxes per CTA: the 272-byte formats keep two with 128-token tiles, which leaves room for a deeper stage ring
+// boxes per CTA: the 272-byte formats keep two with 128-token tiles, which leaves room for a deeper stage ring; tiles of 256 tokens
+// leave room for 72 to 90 KB of boxes beside their two stages
 template <int TN, int QT>
 struct MmqRing {
-  static constexpr int value = (TN >= 128 && MmqStage<QT>::BOX == 272) ? 2 : MmqStage<QT>::RING;
+  static constexpr int value = TN >= 128 && MmqStage<QT>::BOX == 272 ? 2
+                               : TN < 256                              ? MmqStage<QT>::RING
+                                                                       : (MmqStage<QT>::BOX == 240 ? 3 : 4);
 };
 template <int TN, int QT>
 struct MmqStaged {
@@ -514,7 +517,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
   // one-bit phase of the barrier is unambiguous.
   constexpr int KPS = St::KPS;
   static_assert(!MMQ || (STAGES >= 2 && MMQ_GROUPS == 2 * KPS), "see above");
-  static_assert(STAGES * STAGE_BYTES + PRING * MmqStage<QT>::BYTES >= TN * GEMM_BM * 6,
+  // (Packed weights in 256-token tiles are never split along K, see gemm_plan.)
+  static_assert(STAGES * STAGE_BYTES + PRING * MmqStage<QT>::BYTES >= TN * GEMM_BM * (MMQ && TN == 256 ? 2 : 6),
                 "the epilogue stages fp32 partials and a bf16 tile in the ring memory");
   static_assert(STAGES <= 12 && PRING <= 8, "barrier block layout");
   uint64_t* packed_full = reinterpret_cast<uint64_t*>(bars + 256);  // [PRING <= 8] (STAGED only)
@@ -1108,16 +1112,22 @@ struct GemmPlan {
 extern int g_oxb_cluster_splitk;  // 1 = split-K through clusters / distributed shared memory (default)
 extern int g_oxb_gemm_prefill_tn;  // 0 = pick the token tile of prefill-sized calls by wave count, 128 / 256 = force
 
-// packed: the packed-weight kernel (one CTA per SM, 128-token tiles at most).  cluster_ok < 0: follow g_oxb_cluster_splitk.  max_ctas > 0 bounds tiles*splits (kernels whose CTAs wait
+// packed: the packed-weight kernel (one CTA per SM).  cluster_ok < 0: follow g_oxb_cluster_splitk.  max_ctas > 0 bounds tiles*splits (kernels whose CTAs wait
 // for CTAs of other GPUs must be resident all at once).
 inline GemmPlan gemm_plan(int T, int N, int K, int splits_hint, int sm_count, int cluster_ok = -1, int max_ctas = 0,
                           bool packed = false, int groups = 1) {
   GemmPlan p;
   if (cluster_ok < 0) cluster_ok = g_oxb_cluster_splitk;
   p.tn = T <= 16 ? 16 : T <= 32 ? 32 : T <= 64 ? 64 : T <= 128 ? 128 : 256;
-  if (packed && p.tn > 128) p.tn = 128;  // packed weights: 128-token tiles at most (TMEM holds the accumulator and the A ring)
   p.n_tiles = (N + GEMM_BM - 1) / GEMM_BM;
-  if (T > 256 && sm_count > 0) {
+  if (packed && T > 128) {
+    // A k-block costs the decoders about as long as the products of 256 tokens take (550 and 512 cycles), so a tile of 256 tokens
+    // takes little longer than one of 128 and decodes half as often: it is taken wherever it saves a wave.
+    const int sms = sm_count > 0 ? sm_count : 148;
+    const long long w256 = ((long long)p.n_tiles * groups * ((T + 255) / 256) + sms - 1) / sms;
+    const long long w128 = ((long long)p.n_tiles * groups * ((T + 127) / 128) + sms - 1) / sms;
+    p.tn = w256 < w128 ? 256 : 128;
+  } else if (T > 256 && sm_count > 0) {
     // Prefill-sized calls run one CTA per SM in waves; a nearly empty last wave costs a whole tile time.
     // 128-token tiles take half as long as 256-token ones, so compare the wave counts in half-tile units.
     const long long w256 = ((long long)p.n_tiles * groups * ((T + 255) / 256) + sm_count - 1) / sm_count * 2;
@@ -1126,7 +1136,7 @@ inline GemmPlan gemm_plan(int T, int N, int K, int splits_hint, int sm_count, in
   }
   p.t_tiles = (T + p.tn - 1) / p.tn;
   const int kb_total = (K + GEMM_BK - 1) / GEMM_BK;
-  int splits = splits_hint;
+  int splits = packed && p.tn == 256 ? 1 : splits_hint;
   if (splits <= 0) {
     // Among the admissible split counts pick the one with the smallest critical path: k-blocks
     // streamed by the busiest SM plus a fixed cost per split for the reduction.  Without clusters
@@ -1233,6 +1243,7 @@ int gemm_launch(const CUtensorMap& tmW, const CUtensorMap& tmX, __nv_bfloat16* Y
     configured[dev] = true;
   }
   int splits = p.splits;
+  if (QT != QT_BF16 && TN == 256 && splits != 1) return (int)cudaErrorInvalidConfiguration;  // (no room for partials)
   if (p.cluster) {
     const int mc = gemm_max_cluster<TN, QT>();
     if (splits > mc) splits = mc;
@@ -1268,7 +1279,8 @@ int gemm_launch_mmq(const CUtensorMap& tmX, __nv_bfloat16* Y, const float* bias,
     case 32: return gemm_launch<32, QT>(tmW, tmX, Y, bias, N, T, K, ldY, p, ws, counters, epi_mode, ar, stream, qw, gr, groups);
     case 64: return gemm_launch<64, QT>(tmW, tmX, Y, bias, N, T, K, ldY, p, ws, counters, epi_mode, ar, stream, qw, gr, groups);
     case 128: return gemm_launch<128, QT>(tmW, tmX, Y, bias, N, T, K, ldY, p, ws, counters, epi_mode, ar, stream, qw, gr, groups);
-    default: return (int)cudaErrorInvalidConfiguration;  // packed weights are planned with 128-token tiles at most
+    case 256: return gemm_launch<256, QT>(tmW, tmX, Y, bias, N, T, K, ldY, p, ws, counters, epi_mode, ar, stream, qw, gr, groups);
+    default: return (int)cudaErrorInvalidConfiguration;
   }
 }
 

@@ -421,7 +421,8 @@ OXB_API int oxb_gemm_grouped_rows(const void* X, int rows_cap, const void* W, in
   // (128 experts of 1536 x 2048, 640 rows: 385 us with tiles of 128 rows for the 80 that one expert could have had, 136 us,
   // 5.9 TB/s, with tiles of 16.)
   const long long avg = ((long long)rows_cap + groups - 1) / groups;
-  const int rows = 2 * avg < max_rows ? (int)(2 * avg) : max_rows;
+  int rows = 2 * avg < max_rows ? (int)(2 * avg) : max_rows;
+  if (packed && avg <= 96 && rows > 128) rows = 128;  // (most groups fit a tile of 128: one of 256 would only be emptier)
   GemmPlan p = gemm_plan(rows, N, K, 0, sm_count(), 1, 0, packed, groups);
   if (p.splits > 1 && !p.cluster) p = gemm_plan(rows, N, K, 1, sm_count(), 1, 0, packed, groups);
   p.t_tiles = (int)gathered_tiles(rows_cap, groups, max_rows, p.tn);

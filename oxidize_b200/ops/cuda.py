@@ -66,9 +66,9 @@ class KernelOptions:
     gemv_wide: bool = False  # ... also for wide, short matrices (K >= 2N), where the split-K tensor-core kernel is faster
     ar_ll_min_world: int = 2  # rank counts from which the fused all-reduce uses the two-shot exchange
     # Packed-weight calls with more tokens than this decode the matrix to a bf16 staging buffer once and run the bf16
-    # GEMM on it (every token tile of the fused kernel decodes the weight tile again: past ~900 tokens decoding once
-    # wins, 1.4x at 2304 tokens); 0 = always the fused kernel.
-    mmq_max_tokens: int = 1024
+    # GEMM on it (every token tile of the fused kernel decodes the weight tile again); 0 = always the fused kernel,
+    # -1 = by encoding (cuda_quant.DECODE_ABOVE).
+    mmq_max_tokens: int = -1
     # Checked mode: the op layer's scratch buffers (split-K partials and tickets, split-KV partials, decode staging) sit
     # between canary bands that ``verify_guards()`` checks (``LLM.step`` does so after every step, the kernel tests
     # after every test).  Costs a device synchronisation per check: for debugging, not for serving.
@@ -510,9 +510,11 @@ def attn_splits(B: int, nkv: int, mtiles: int, max_seq_len: int, sms: int, per_s
     return max(1, min(want, cap, 16))
 
 
-# Sequences that feed at least PREFILL_ROWS rows in a step take the tcgen05 kernel: it runs 256 (token, head) rows of a key head to
-# a CTA, the other 16.  8 sequences over 1000 rows, 32 heads / 8: 48 rows 35 against 80 us, 16 rows 33 against 33.
-PREFILL_ROWS = 32
+# Long portions take the tcgen05 kernel, which runs 256 (token, head) rows of a key head to a CTA, the other 16 and those split along
+# the keys.  From PREFILL_SURE rows on it is ahead over any context (256 rows over 1000 / 8000, 32 heads / 8: 38 / 176 us against
+# 61 / 281; over none 17 against 27).  Fewer rows leave SMs idle that the other's splits would use (one sequence of 64 over 8000:
+# 169 against 85 us; four of them 214 against 411): there the estimates decide, 1.3 us per 64 keys and wave of CTAs, and 100 TFLOP/s.
+PREFILL_ROWS, PREFILL_SURE = 32, 192
 PREFILL_MAX_PAGES = 1 << 14  # ... their pages, where they have to be converted to bf16 first, up to this many in a step
 
 
@@ -521,10 +523,16 @@ def _long_portions(q, kv, layer, meta) -> bool:
     lens = getattr(meta, "host_lens", None)
     if not lens or len(lens) != meta.seq_lens.shape[0] or kv.page_size != 16 or q.dtype != torch.bfloat16:
         return False
-    pages = [(c + 15) // 16 for n, c in lens if n >= PREFILL_ROWS]
-    if not pages or (kv.dtype_name != "bf16" and sum(pages) > PREFILL_MAX_PAGES):
+    long = [(n, c) for n, c in lens if n >= PREFILL_ROWS]
+    nq, hd, nkv = q.shape[1], q.shape[2], kv.spec.heads(layer)
+    if not long or (kv.dtype_name != "bf16" and sum((c + 15) // 16 for _, c in long) > PREFILL_MAX_PAGES):
         return False
-    return bool(lib().oxb_paged_prefill_supported(q.shape[2], q.shape[1], kv.spec.heads(layer)))
+    if max(n for n, _ in long) < PREFILL_SURE:
+        ctas = sum(-(-n * nq // 256) for n, _ in long)
+        here = 1.3 * -(-ctas // sm_count(q.device)) * (max(c for _, c in long) / 64 + 6) + 6
+        if here > sum(4e-8 * nq * hd * n * (c - n / 2) for n, c in long) + 8:
+            return False
+    return bool(lib().oxb_paged_prefill_supported(hd, nq, nkv))
 
 
 def _paged_prefill(q, kv, layer, meta, scale, window, sink, out, out_scale, gate, gate_per_value) -> None:

@@ -3,8 +3,7 @@ block-scaled fp8) on the GPU.
 
 Everything goes through ``oxb_gemm_quant``.  Calls with one or two tokens take the dp4a GEMV
 (``csrc/gemv_quant.cuh``: int8 activations, the packed bytes go straight into the arithmetic); larger
-batches the tcgen05 GEMM whose producer warps decode the blocks into the swizzled shared-memory
-operand tile.  Either way the weights are read from HBM once, in their packed form.  Formats without a
+batches the tcgen05 GEMM whose producer warps decode the blocks into tensor memory.  Either way the weights are read from HBM once, in their packed form.  Formats without a
 fused decoder (Q5_K, Q4_1 …), or a K that is not a multiple of 64, are decoded to a bf16 staging
 buffer first.
 """
@@ -16,6 +15,18 @@ from . import cuda as C
 
 FUSED_TYPES = {"Q4_K": 5, "Q6_K": 7, "Q8_0": 3, "Q4_0": 4, "NVFP4": 8}
 QT_FP8B = 9
+# Tokens above which a matrix is decoded once instead of by every token tile (0: never).  28672 x 4096, fused / decoded once, us,
+# at 1024, 2048 and 4096 tokens: Q4_K 224 / 320, 404 / 492, 775 / 835; NVFP4 239 / 517, 431 / 685, 825 / 1021; Q8_0 252 / 318,
+# 456 / 488, 861 / 836; Q6_K 290 / 316, 523 / 485, 984 / 833 (even at about 1300).  Rows that are not whole super-blocks of 256 are
+# read without staging, by every tile: once from 1024 tokens on.
+DECODE_ABOVE = {"Q4_K": 0, "NVFP4": 0, "Q8_0": 3072, "Q6_K": 1280}
+DECODE_ABOVE_ELSE = 1024
+
+
+def decode_above(qtype: str, k: int) -> int:
+    if C.mmq_max_tokens >= 0:
+        return C.mmq_max_tokens
+    return DECODE_ABOVE.get(qtype, DECODE_ABOVE_ELSE) if k % 256 == 0 else DECODE_ABOVE_ELSE
 
 
 def _launch(x, data_ptr, qt, row_bytes, scales_ptr, scale_ld, out_view, bias, ld_out, N, K):
@@ -29,7 +40,8 @@ def _launch(x, data_ptr, qt, row_bytes, scales_ptr, scale_ld, out_view, bias, ld
 
 def linear_quant(x, p, out_view, bias, ld_out):
     n, k = p.shape
-    staged_ok = C.mmq_max_tokens > 0 and x.shape[0] > C.mmq_max_tokens and n * k <= (1 << 28)
+    limit = decode_above(p.qtype, k)
+    staged_ok = 0 < limit < x.shape[0] and n * k <= (1 << 28)
     if p.qtype in FUSED_TYPES and k % 64 == 0 and not staged_ok:
         row_bytes = p.data.stride(0) * p.data.element_size()
         return _launch(x, p.data.data_ptr(), FUSED_TYPES[p.qtype], row_bytes, None, 0, out_view, bias, ld_out, n, k)
