@@ -32,20 +32,28 @@ __device__ __forceinline__ int dp4a_us(uint32_t a, uint32_t b, int c) {  // a un
   return d;
 }
 
+// Loads of packed bytes, from shared memory or from global (read-only) memory
+template <bool SHARED, class T>
+__device__ __forceinline__ T gv_ld(const T* p) {
+  if constexpr (SHARED) return *p;
+  else return __ldg(p);
+}
 // 16 bytes from an address that is only 2-byte aligned: aligned words + funnel shift.
+template <bool SHARED>
 __device__ __forceinline__ void ld16_align2(const uint8_t* p, uint32_t (&o)[4]) {
   const uintptr_t a = reinterpret_cast<uintptr_t>(p);
   const uint32_t* w = reinterpret_cast<const uint32_t*>(a & ~uintptr_t(3));
   const uint32_t sh = (uint32_t)(a & 2) * 8;
-  const uint32_t x0 = __ldg(w), x1 = __ldg(w + 1), x2 = __ldg(w + 2), x3 = __ldg(w + 3);
-  const uint32_t x4 = sh ? __ldg(w + 4) : 0u;
+  const uint32_t x0 = gv_ld<SHARED>(w), x1 = gv_ld<SHARED>(w + 1), x2 = gv_ld<SHARED>(w + 2), x3 = gv_ld<SHARED>(w + 3);
+  const uint32_t x4 = sh ? gv_ld<SHARED>(w + 4) : 0u;
   o[0] = __funnelshift_r(x0, x1, sh);
   o[1] = __funnelshift_r(x1, x2, sh);
   o[2] = __funnelshift_r(x2, x3, sh);
   o[3] = __funnelshift_r(x3, x4, sh);
 }
+template <bool SHARED>
 __device__ __forceinline__ float ld_half_raw(const uint8_t* p) {
-  return __half2float(__ushort_as_half(__ldg(reinterpret_cast<const unsigned short*>(p))));
+  return __half2float(__ushort_as_half(gv_ld<SHARED>(reinterpret_cast<const unsigned short*>(p))));
 }
 
 // (scale, min) pair j of a Q4_K block whose 12 packed bytes are the words s0 s1 s2
@@ -109,7 +117,7 @@ struct GvFrag {
   bool live;
 };
 
-template <int QT>
+template <int QT, bool SHARED = false>
 __device__ __forceinline__ void gv_load(const uint8_t* rowp, int it, int lane, int K, GvFrag<QT>& f) {
   f.live = false;
   if constexpr (QT == QT_Q4_K) {
@@ -117,8 +125,8 @@ __device__ __forceinline__ void gv_load(const uint8_t* rowp, int it, int lane, i
     if (sb * 256 >= K) return;
     const int l8 = lane & 7;
     const uint8_t* b = rowp + (size_t)sb * 144;
-    const uint4 hdr = __ldg(reinterpret_cast<const uint4*>(b));
-    const uint4 qv = __ldg(reinterpret_cast<const uint4*>(b + 16 + 16 * l8));
+    const uint4 hdr = gv_ld<SHARED>(reinterpret_cast<const uint4*>(b));
+    const uint4 qv = gv_ld<SHARED>(reinterpret_cast<const uint4*>(b + 16 + 16 * l8));
     f.a[0] = hdr.x; f.a[1] = hdr.y; f.a[2] = hdr.z; f.a[3] = hdr.w;
     f.b[0] = qv.x; f.b[1] = qv.y; f.b[2] = qv.z; f.b[3] = qv.w;
     f.live = true;
@@ -127,26 +135,26 @@ __device__ __forceinline__ void gv_load(const uint8_t* rowp, int it, int lane, i
     if (sb * 256 >= K) return;
     const int l8 = lane & 7, h = l8 >> 2, i = l8 & 3, q0 = i >> 1, lr = (i & 1) * 16;
     const uint8_t* b = rowp + (size_t)sb * 210;
-    ld16_align2(b + h * 64 + 16 * i, f.a);
-    ld16_align2(b + 128 + h * 32 + lr, f.b);
+    ld16_align2<SHARED>(b + h * 64 + 16 * i, f.a);
+    ld16_align2<SHARED>(b + 128 + h * 32 + lr, f.b);
     const int8_t* scp = reinterpret_cast<const int8_t*>(b + 192) + h * 8 + (i & 1) + 2 * q0;
-    const float d = ld_half_raw(b + 208);
-    f.dlo = d * (float)__ldg(scp);
-    f.dhi = d * (float)__ldg(scp + 4);
+    const float d = ld_half_raw<SHARED>(b + 208);
+    f.dlo = d * (float)gv_ld<SHARED>(scp);
+    f.dhi = d * (float)gv_ld<SHARED>(scp + 4);
     f.live = true;
   } else if constexpr (QT == QT_Q8_0) {
     const int blk = it * 16 + (lane >> 1), hh = lane & 1;
     if (blk * 32 >= K) return;
     const uint8_t* b = rowp + (size_t)blk * 34;
-    ld16_align2(b + 2 + 16 * hh, f.a);
-    f.d = ld_half_raw(b);
+    ld16_align2<SHARED>(b + 2 + 16 * hh, f.a);
+    f.d = ld_half_raw<SHARED>(b);
     f.live = true;
   } else if constexpr (QT == QT_Q4_0) {
     const int blk = it * 32 + lane;
     if (blk * 32 >= K) return;
     const uint8_t* b = rowp + (size_t)blk * 18;
-    ld16_align2(b + 2, f.a);
-    f.d = ld_half_raw(b);
+    ld16_align2<SHARED>(b + 2, f.a);
+    f.d = ld_half_raw<SHARED>(b);
     f.live = true;
   }
 }
@@ -352,9 +360,216 @@ gemv_quant_kernel(const uint8_t* __restrict__ W, size_t row_bytes, const __nv_bf
   }
 }
 
+// The same product as a stream: every warp owns a ring of segments of row pairs in shared memory that bulk copies fill, so how many
+// bytes are in flight does not depend on registers or on where a warp is in its arithmetic, and as the weights are static the
+// first rings (up to 105 KB per SM) are requested before the kernel waits for its activations.  One CTA of 16 warps per SM in
+// less than half of its shared memory: the next product's CTA fits beside it and has its rings filled when its turn comes.
+// 28672 x 4096, one token, launch included: Q4_K 28.7 us before, 24.6 now; Q6_K 49 and 39; Q8_0 57 and 41.
+// gemv_quant_kernel stays for rows that are not whole warp iterations or not on 16-byte boundaries, and for more than two tokens.
+constexpr int GS_WARPS = 16, GS_ROWS = 2, GS_WARP_RING = 6720;
+template <int QT>
+struct GvSeg {
+  static constexpr int VALUES = QT == QT_Q8_0 ? 1024 : 2048;  // of one row
+  static constexpr int BYTES = QT == QT_Q4_K ? VALUES / 256 * 144 : QT == QT_Q6_K ? VALUES / 256 * 210 : VALUES / 32 * 34;
+  static constexpr int STAGES = GS_WARP_RING / (GS_ROWS * BYTES);
+  static constexpr int SPAN = QT == QT_Q4_K ? 2048 : GvSpan<QT>::VALUES;  // values of one warp iteration
+  static_assert(STAGES >= 2 && BYTES % 16 == 0, "ring layout");
+};
+template <int QT, int TB>
+size_t gs_smem_bytes(int K) {  // (16 bytes past the rings: an unaligned read may touch the word after a segment)
+  return (gv_smem_bytes(TB, K) + 15) / 16 * 16 + (size_t)GS_WARPS * GvSeg<QT>::STAGES * GS_ROWS * GvSeg<QT>::BYTES + 16;
+}
+
+// Q4_K in the stream: a lane takes a whole group of 64 values (32 bytes: two sub-blocks, one in the low and one in the high nibbles) of
+// one of eight super-blocks, so that their scales are unpacked once per 64 values (gv_load / gv_dot: per 32); the kernel is
+// bound by instructions otherwise (28672 x 4096: 34 us with those, against 66 MB).  The activations are shared by the rows.
+template <int TB, int ROWS>
+__device__ __forceinline__ void gs_dot_q4k(const uint8_t* seg, int k0, int lane, const GvAct& act, float (&acc)[ROWS][TB]) {
+  const int sb = lane >> 2, c = lane & 3;
+  uint32_t q[ROWS][8];
+  float ds0[ROWS], ds1[ROWS], dm0[ROWS], dm1[ROWS];
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) {
+    const uint8_t* b = seg + r * GvSeg<QT_Q4_K>::BYTES + sb * 144;
+    const uint4 hdr = *reinterpret_cast<const uint4*>(b);
+    const uint4 qa = *reinterpret_cast<const uint4*>(b + 16 + 32 * c), qb = *reinterpret_cast<const uint4*>(b + 32 + 32 * c);
+    q[r][0] = qa.x; q[r][1] = qa.y; q[r][2] = qa.z; q[r][3] = qa.w;
+    q[r][4] = qb.x; q[r][5] = qb.y; q[r][6] = qb.z; q[r][7] = qb.w;
+    const float d = __half2float(__ushort_as_half((unsigned short)(hdr.x & 0xFFFF)));
+    const float dmin = __half2float(__ushort_as_half((unsigned short)(hdr.x >> 16)));
+    const int sh = 16 * (c & 1);  // two scales / minima, one per byte
+    const uint32_t y = hdr.y >> sh, z = hdr.z >> sh, w = hdr.w >> sh;
+    const uint32_t sc2 = c < 2 ? y & 0x3F3F : (w & 0x0F0F) | ((y & 0xC0C0) >> 2);
+    const uint32_t m2 = c < 2 ? z & 0x3F3F : ((w >> 4) & 0x0F0F) | ((z & 0xC0C0) >> 2);
+    ds0[r] = d * (float)(sc2 & 0xFF);
+    ds1[r] = d * (float)((sc2 >> 8) & 0xFF);
+    dm0[r] = dmin * (float)(m2 & 0xFF);
+    dm1[r] = dmin * (float)((m2 >> 8) & 0xFF);
+  }
+  const int x0 = k0 + sb * 256;
+#pragma unroll
+  for (int t = 0; t < TB; ++t) {
+    const uint4* xl = reinterpret_cast<const uint4*>(act.q + (size_t)t * act.K + x0 + 32 * c);  // (gv_act_pos: low nibbles' values first)
+    const uint4 l0 = xl[0], l1 = xl[1], h0 = xl[8], h1 = xl[9];
+    const uint32_t lo[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w}, hi[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+    const float2 dx = *reinterpret_cast<const float2*>(act.d + (size_t)t * (act.K >> 5) + ((x0 + 64 * c) >> 5));
+    const short4 s = *reinterpret_cast<const short4*>(act.s16 + (size_t)t * (act.K >> 4) + ((x0 + 64 * c) >> 4));
+    const float s0 = (float)(s.x + s.y), s1 = (float)(s.z + s.w);
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      int slo = 0, shi = 0;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) {
+        slo = dp4a_ss(q[r][w] & 0x0F0F0F0Fu, lo[w], slo);
+        shi = dp4a_ss((q[r][w] >> 4) & 0x0F0F0F0Fu, hi[w], shi);
+      }
+      acc[r][t] += dx.x * (ds0[r] * (float)slo - dm0[r] * s0) + dx.y * (ds1[r] * (float)shi - dm1[r] * s1);
+    }
+  }
+}
+
+template <int QT, int TB>
+__global__ void __launch_bounds__(GS_WARPS * 32)
+gemv_stream_kernel(const uint8_t* __restrict__ W, size_t row_bytes, const __nv_bfloat16* __restrict__ X, int ldX,
+                   __nv_bfloat16* __restrict__ Y, int ldY, const float* __restrict__ bias, int T, int N, int K, int add_into) {
+  using Seg = GvSeg<QT>;
+  constexpr int D = Seg::STAGES, SLOT = GS_ROWS * Seg::BYTES;
+  extern __shared__ __align__(16) uint8_t gv_smem[];
+  __shared__ uint64_t full[GS_WARPS][D];
+  __shared__ volatile int abort_flag;
+  int8_t* xq = reinterpret_cast<int8_t*>(gv_smem);
+  float* xd = reinterpret_cast<float*>(gv_smem + (size_t)TB * K);
+  short* xs = reinterpret_cast<short*>(gv_smem + (size_t)TB * K + (size_t)TB * (K >> 5) * 4);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint8_t* ring = gv_smem + (gv_smem_bytes(TB, K) + 15) / 16 * 16 + (size_t)warp * D * SLOT;
+  // row pairs gw, gw + nw, ...: what is left over of N goes to different SMs
+  const int gw = warp * gridDim.x + blockIdx.x, nw = gridDim.x * GS_WARPS, pairs = (N + GS_ROWS - 1) / GS_ROWS;
+  const int segs = (K + Seg::VALUES - 1) / Seg::VALUES;
+  pdl_launch_dependents();
+  if (threadIdx.x == 0) abort_flag = 0;
+  int f_pair = gw, f_seg = 0;  // next segment to fetch
+  auto fetch = [&](int slot) {
+    if (f_pair >= pairs) return;
+    if (lane == 0) {
+      const uint32_t left = (uint32_t)(row_bytes - (size_t)f_seg * Seg::BYTES);
+      const uint32_t bytes = left < (uint32_t)Seg::BYTES ? left : (uint32_t)Seg::BYTES;
+      mbar_expect_tx(&full[warp][slot], GS_ROWS * bytes);
+#pragma unroll
+      for (int r = 0; r < GS_ROWS; ++r) {
+        const int row = min(GS_ROWS * f_pair + r, N - 1);  // a row past the end is the last one again, computed and dropped
+        bulk_load(ring + slot * SLOT + r * Seg::BYTES, W + (size_t)row * row_bytes + (size_t)f_seg * Seg::BYTES, bytes, &full[warp][slot]);
+      }
+    }
+    if (++f_seg == segs) {
+      f_seg = 0;
+      f_pair += nw;
+    }
+  };
+  if (lane == 0) {
+    for (int i = 0; i < D; ++i) mbar_init(&full[warp][i], 1);
+    mbar_fence_init();
+  }
+  __syncwarp();
+#pragma unroll 1
+  for (int i = 0; i < D; ++i) fetch(i);
+  pdl_wait();  // the activations come from the upstream kernel
+  gv_quantize_x<QT, TB>(X, ldX, T, K, xq, xd, xs);
+  __syncthreads();
+  const GvAct act{xq, xd, xs, K};
+  int slot = 0;
+  uint32_t ph = 0;
+  bool ok = true;
+  for (int p = gw; p < pairs && ok; p += nw) {
+    float acc[GS_ROWS][TB];
+#pragma unroll
+    for (int r = 0; r < GS_ROWS; ++r)
+#pragma unroll
+      for (int t = 0; t < TB; ++t) acc[r][t] = 0.f;
+    for (int sg = 0; sg < segs; ++sg) {
+      ok = __all_sync(0xffffffffu, mbar_wait_bounded(&full[warp][slot], ph, &abort_flag, OXB_TIMEOUT_TMA_FULL, blockIdx.x));
+      if (!ok) break;
+      const uint8_t* seg = ring + slot * SLOT;
+      if constexpr (QT == QT_Q4_K) {
+        gs_dot_q4k<TB, GS_ROWS>(seg, sg * Seg::VALUES, lane, act, acc);
+      } else {
+        // (gv_load and gv_dot count iterations from the start of the row)
+        constexpr int PER = Seg::VALUES / Seg::SPAN;
+        const uint8_t* rowp = seg - (size_t)sg * Seg::BYTES;
+        GvFrag<QT> fr[PER][GS_ROWS];
+#pragma unroll
+        for (int g = 0; g < PER; ++g)
+#pragma unroll
+          for (int r = 0; r < GS_ROWS; ++r) gv_load<QT, true>(rowp + r * Seg::BYTES, sg * PER + g, lane, K, fr[g][r]);
+#pragma unroll
+        for (int g = 0; g < PER; ++g)
+#pragma unroll
+          for (int r = 0; r < GS_ROWS; ++r) gv_dot<QT, TB>(fr[g][r], sg * PER + g, lane, act, acc[r]);
+      }
+      __syncwarp();
+      fetch(slot);
+      if (++slot == D) {
+        slot = 0;
+        ph ^= 1;
+      }
+    }
+    if (!ok) break;
+#pragma unroll
+    for (int r = 0; r < GS_ROWS; ++r) {
+      const int row = GS_ROWS * p + r;
+#pragma unroll
+      for (int t = 0; t < TB; ++t) {
+        float v = warp_sum(acc[r][t]);
+        if (lane == 0 && row < N && t < T) {
+          if (bias != nullptr) v += bias[row];
+          __nv_bfloat16* dst = Y + (size_t)t * ldY + row;
+          if (add_into) v += __bfloat162float(*dst);
+          *dst = __float2bfloat16(v);
+        }
+      }
+    }
+  }
+  if (!ok) {
+    // a wait gave up: give copies that may still be in flight time to land before the CTA exits
+    for (int i = 0; i < 64; ++i) __nanosleep(2000);
+  }
+}
+
+// Whether the stream covers a product: whole warp iterations, row segments on 16-byte boundaries, shared memory.
+template <int QT, int TB>
+bool gemv_stream_covers(const uint8_t* W, size_t row_bytes, int K) {
+  return K % GvSeg<QT>::SPAN == 0 && row_bytes == (size_t)GvSeg<QT>::BYTES * K / GvSeg<QT>::VALUES && row_bytes % 16 == 0 &&
+         (reinterpret_cast<uintptr_t>(W) & 15) == 0 && gs_smem_bytes<QT, TB>(K) <= 220 * 1024;
+}
+
+template <int QT, int TB>
+int gemv_stream_launch(const uint8_t* W, size_t row_bytes, const __nv_bfloat16* X, int ldX, __nv_bfloat16* Y, int ldY,
+                       const float* bias, int T, int N, int K, int add_into, int sm_count, cudaStream_t stream) {
+  const size_t smem = gs_smem_bytes<QT, TB>(K);
+  auto kfn = gemv_stream_kernel<QT, TB>;
+  static size_t configured[64] = {0};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) return (int)cudaErrorInvalidDevice;
+  if (smem > configured[dev]) {
+    cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    configured[dev] = smem;
+  }
+  int grid = (N + GS_WARPS * GS_ROWS - 1) / (GS_WARPS * GS_ROWS);
+  if (grid > sm_count) grid = sm_count;
+  cudaError_t le = oxb_launch(kfn, dim3(grid), dim3(GS_WARPS * 32), smem, stream, W, row_bytes, X, ldX, Y, ldY, bias, T, N, K, add_into);
+  if (le != cudaSuccess) return (int)le;
+  OXB_CHECK_LAUNCH();
+  return 0;
+}
+
 template <int QT, int TB>
 int gemv_quant_launch(const uint8_t* W, size_t row_bytes, const __nv_bfloat16* X, int ldX, __nv_bfloat16* Y, int ldY,
                       const float* bias, int T, int N, int K, int add_into, int sm_count, cudaStream_t stream) {
+  if constexpr (TB <= 2 && QT != QT_Q4_0) {
+    if (gemv_stream_covers<QT, TB>(W, row_bytes, K))
+      return gemv_stream_launch<QT, TB>(W, row_bytes, X, ldX, Y, ldY, bias, T, N, K, add_into, sm_count, stream);
+  }
   constexpr int RPW = TB <= 2 ? 2 : 1;
   const size_t smem = gv_smem_bytes(TB, K);
   auto kfn = gemv_quant_kernel<QT, TB, RPW>;
