@@ -1,0 +1,140 @@
+"""Kernels whose tiles follow the size of a call, at the edges of those tiles, against plain statements of the same op."""
+import pytest
+import torch
+
+from oxidize_b200.engine.kv_pool import KVCache, KVCacheSpec
+from oxidize_b200.models.transformer import BatchMeta
+from oxidize_b200.models.weights import qtensor_from_dense
+from oxidize_b200.ops import ref
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def C():
+    from oxidize_b200.ops import cuda as C
+
+    C.lib()
+    return C
+
+
+def _off(a, b):
+    a, b = a.double().cpu(), b.double().cpu()
+    return float((a - b).norm() / b.norm())
+
+
+def _check_status(C):
+    torch.cuda.synchronize()
+    assert C.status() == (0, 0, 0)
+
+
+# ------------------------------------------------------------------------------------------------- attention
+def _step(kvd, hd, nq, nkv, lens, seed=0):
+    """Cache (pages in random order, a page past each sequence's own), step and queries of (rows fed, context) sequences."""
+    gen = torch.Generator().manual_seed(seed)
+    need = [(c + 15) // 16 for _, c in lens]
+    cpu = KVCache(KVCacheSpec(1, nkv, hd, 16, kvd), sum(need) + 2, torch.device("cpu"))
+    order = torch.randperm(sum(need) + 2, generator=gen).tolist()
+    tables, at = [], 0
+    for n, (_, c) in zip(need, lens):
+        tables.append(order[at : at + n] + [0] * (max(need) + 1 - n))
+        at += n
+        slots = torch.tensor([tables[-1][p // 16] * 16 + p % 16 for p in range(c)], dtype=torch.int32)
+        k, v = (torch.randn(c, nkv, hd, generator=gen).bfloat16().float() for _ in range(2))
+        ref.kv_write(cpu, 0, k, v, slots)
+    starts = [sum(n for n, _ in lens[:i]) for i in range(len(lens) + 1)]
+    ints = lambda v: torch.tensor(v, dtype=torch.int32)  # noqa: E731
+    meta = BatchMeta(None, None, None, ints(starts), ints([c for _, c in lens]), ints(tables), None, max(n for n, _ in lens),
+                     max(c for _, c in lens), len(lens))
+    gpu = KVCache(cpu.spec, cpu.num_blocks, torch.device("cuda"))
+    gpu.data = [d.cuda() for d in cpu.data]
+    gpu.scales = [None if s is None else s.cuda() for s in cpu.scales]
+    on_gpu = BatchMeta(None, None, None, meta.query_start.cuda(), meta.seq_lens.cuda(), meta.block_tables.cuda(), None, meta.max_query_len,
+                       meta.max_seq_len, len(lens), host_lens=list(lens))
+    q = torch.randn(starts[-1], nq, hd, generator=gen).bfloat16()
+    return cpu, meta, gpu, on_gpu, q
+
+
+LONG = [(200, 200), (64, 300), (1, 70), (33, 33), (3, 18), (257, 450)]  # long ones, and short ones that the other kernel takes
+
+
+@pytest.mark.parametrize("kvd,hd,nq,nkv,lens,window", [
+    ("bf16", 128, 8, 2, LONG, 0), ("bf16", 64, 4, 4, LONG, 0), ("bf16", 128, 7, 1, LONG, 0), ("bf16", 128, 12, 2, [(192, 193)], 0),
+    ("bf16", 128, 16, 1, [(224, 1000)], 0), ("bf16", 128, 8, 2, LONG, 50), ("bf16", 64, 4, 2, [(200, 400)], 200),
+    ("f16", 128, 8, 2, LONG, 0), ("q8", 128, 8, 2, LONG, 0), ("q4", 128, 8, 2, LONG, 0), ("q8", 64, 4, 1, LONG, 90), ("q4", 64, 4, 2, LONG, 0)])
+def test_long_portions(C, kvd, hd, nq, nkv, lens, window):
+    cpu, meta, gpu, on_gpu, q = _step(kvd, hd, nq, nkv, lens)
+    got = C.paged_attention(q.cuda(), gpu, 0, on_gpu, hd ** -0.5, window)
+    _check_status(C)
+    want = ref.paged_attention(q.float(), cpu, 0, meta, hd ** -0.5, window)
+    # outputs are rounded to bf16 (2e-3 at most), and f16 and quantized rows on their way in (as much again, keys and values)
+    assert _off(got, want) < (2.5e-3 if kvd == "bf16" else 6e-3)
+    assert torch.isfinite(got.float()).all()
+
+
+def test_long_portion_with_sink_gate_and_a_wider_output(C):
+    cpu, meta, gpu, on_gpu, q = _step("bf16", 128, 8, 2, LONG)
+    T = q.shape[0]
+    sink, gate = torch.randn(8), torch.randn(T, 8 * 128).bfloat16()
+    wide = torch.full((T, 8 * 128 + 10), 7.0, dtype=torch.bfloat16, device="cuda")
+    C.paged_attention(q.cuda(), gpu, 0, on_gpu, 128 ** -0.5, sink=sink.cuda(), out=wide[:, 2 : 2 + 8 * 128], gate=gate.cuda(),
+                      gate_per_value=True)
+    other = C.paged_attention(q.cuda(), gpu, 0, on_gpu, 128 ** -0.5, splits=1, sink=sink.cuda(), gate=gate.cuda(), gate_per_value=True)
+    _check_status(C)
+    assert _off(wide[:, 2 : 2 + 8 * 128], other.reshape(T, -1)) < 6e-3  # (two roundings to bf16, probabilities of the other's to bf16 too)
+    assert (wide[:, :2] == 7).all() and (wide[:, 2 + 8 * 128 :] == 7).all()
+
+
+@pytest.mark.parametrize("kvd", ["q8", "q4"])
+@pytest.mark.parametrize("hd,nq,nkv,lens", [(128, 8, 2, [(1, 1), (1, 16), (1, 17), (5, 333), (1, 2000)]), (64, 7, 7, [(1, 40), (3, 3)]),
+                                            (64, 32, 2, [(1, 500), (4, 64)])])
+def test_quantized_pages_in_fragments(C, kvd, hd, nq, nkv, lens):
+    cpu, meta, gpu, on_gpu, q = _step(kvd, hd, nq, nkv, lens)
+    want = ref.paged_attention(q.float(), cpu, 0, meta, hd ** -0.5, 0)
+    for splits in (None, 1, 3):
+        got = C.paged_attention(q.cuda(), gpu, 0, on_gpu, hd ** -0.5, splits=splits)
+        _check_status(C)
+        # codes are exact; the output and the scaled probabilities are rounded to bf16
+        assert _off(got, want) < 4e-3
+
+
+# ------------------------------------------------------------------------------------------- packed GEMM
+@pytest.mark.parametrize("qtype", ["Q4_K", "Q6_K", "Q8_0", "NVFP4", "Q4_0"])
+@pytest.mark.parametrize("T,N,K", [(1, 300, 320), (17, 130, 1280), (64, 128, 256), (129, 260, 2816), (256, 20000, 256), (257, 19100, 512),
+                                   (600, 520, 768)])
+def test_packed_gemm_tiles(C, qtype, T, N, K):
+    if qtype in ("Q4_K", "Q6_K") and K % 256:
+        pytest.skip("blocks of 256 values")
+    gen = torch.Generator(device="cuda").manual_seed(T + N)
+    w = qtensor_from_dense((torch.randn(N, K, generator=gen, device="cuda") * 0.05).cpu(), qtype, device="cuda")
+    x = torch.randn(T, K, generator=gen, device="cuda").bfloat16()
+    x[0, : K // 2] = 0
+    C.configure(C.KernelOptions(gemv_max_tokens=0, mmq_max_tokens=0))
+    try:
+        got = C.linear(x, [w])
+        again = C.linear(x, [w])
+    finally:
+        C.configure(C.KernelOptions())
+    _check_status(C)
+    want = x.double() @ C.dequant_rows(w).double().t()  # (decoded value by value, to bf16)
+    assert _off(got, want) < 8e-3  # output, and for the k-quants scales and offsets, rounded to bf16
+    assert torch.equal(got, again)
+
+
+@pytest.mark.parametrize("qtype,N,K", [("BF16", 200, 128), ("Q4_K", 256, 512)])
+@pytest.mark.parametrize("rows", [[0] * 39 + [5], [1] * 40, [0, 300, 0, 17] + [0] * 30 + [16, 33, 1, 0, 128, 129], [2, 700] + [3] * 38])
+def test_grouped_rows_lists(C, qtype, N, K, rows):
+    """Groups with no rows, with rows for several tiles, and more of them than a warp has lanes."""
+    from oxidize_b200.ops import cuda_moe
+
+    E, R = len(rows), sum(rows)
+    gen = torch.Generator(device="cuda").manual_seed(R)
+    dense = torch.randn(E * N, K, generator=gen, device="cuda") * 0.05
+    w = qtensor_from_dense(dense.cpu(), qtype, device="cuda")
+    x = torch.randn(R + 9, K, generator=gen, device="cuda").bfloat16()  # rows past the last group are not touched
+    off = torch.tensor([sum(rows[:i]) for i in range(E + 1)], dtype=torch.int32, device="cuda")
+    got = cuda_moe.gemm_grouped_rows(x, w, off, E, max(rows))
+    _check_status(C)
+    full = (w.data if qtype == "BF16" else C.dequant_rows(w)).double().view(E, N, K)
+    want = torch.cat([x[a:b].double() @ full[e].t() for e, (a, b) in enumerate(zip(off[:-1].tolist(), off[1:].tolist()))])
+    assert _off(got[:R], want) < 8e-3
