@@ -96,6 +96,21 @@ struct AttPage {
   static_assert(SMEM >= ATT_WARPS * 16 * (HD + 2) * 4, "the warps' partial results are merged in the pages' memory");
 };
 
+// mma_bf16_16816 of a tile with NR halves of 8 rows: A and the accumulators hold those halves only (fragments ordered [half of k][half
+// of the rows]).
+template <int NR>
+__device__ __forceinline__ void att_mma(float* d, const uint32_t* a, uint32_t b0, uint32_t b1) {
+  if constexpr (NR == 2) {
+    mma_bf16_16816(d, a, b0, b1);
+  } else {
+    float z0, z1;  // rows 8 to 15: zero times B
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%6,%5,%6}, {%7,%8}, {%0,%1,%9,%9};"
+        : "+f"(d[0]), "+f"(d[1]), "=f"(z0), "=f"(z1)
+        : "r"(a[0]), "r"(a[1]), "r"(0u), "r"(b0), "r"(b1), "f"(0.f));
+  }
+}
+
 // Bring one (K, V) page pair of a kv head into a warp-private stage with cp.async (one warp).
 template <int HD, int MODE>
 __device__ __forceinline__ void load_page(uint8_t* stage, const AttnArgs& a, int blk, int kvh, int lane) {
@@ -207,7 +222,10 @@ __device__ __forceinline__ void attn_merge_rows(const AttnArgs& a, int G, int b,
 // column tiles.  The sums of a key's channel groups are scaled apart, as are the probabilities for the values' groups.
 // (Decoding pages to bf16 rows in shared memory first took 1150 instructions a page and 139 KB, one CTA per SM: at 4 x 25000 q4 rows of
 // 8 heads, 128 wide, 273 us, now 65, of which the copies would take 20; 32 x 640 q8 rows 63 and 25.)
-template <int HD, int MODE>
+// NR: halves of the 16-row tile that hold rows.  A decode step with at most 8 query heads to a key head fills one; the softmax, the
+// scaling of probabilities and half of the accumulators of the other are then left out (and with them 48 registers, which lets a
+// fourth CTA of the q4 form onto an SM).
+template <int HD, int MODE, int NR>
 __global__ void __launch_bounds__(ATT_WARPS * 32, MODE == 0 ? 1 : 3)
 paged_attention_kernel(const AttnArgs a, int G /*q heads per kv head*/) {
   using Page = AttPage<HD, MODE>;
@@ -236,10 +254,10 @@ paged_attention_kernel(const AttnArgs a, int G /*q heads per kv head*/) {
   const bool active = row_base < R;
 
   // rows of this thread: r0 = row_base + g, r1 = r0 + 8
-  int qtok[2], hg[2], qpos[2];
-  bool rvalid[2];
+  int qtok[NR], hg[NR], qpos[NR];
+  bool rvalid[NR];
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
+  for (int i = 0; i < NR; ++i) {
     const int r = row_base + g + 8 * i;
     rvalid[i] = active && r < R;
     qtok[i] = rvalid[i] ? r / G : 0;
@@ -259,10 +277,17 @@ paged_attention_kernel(const AttnArgs a, int G /*q heads per kv head*/) {
   const int first = csplit * ATT_WARPS + warp;  // this warp takes pages first, first+stride, ...
   const int my_pages = n_pages > first ? (n_pages - first + stride - 1) / stride : 0;
 
-  float o[NT][4];
+  float o[NT][2 * NR];
 #pragma unroll
-  for (int nt = 0; nt < NT; ++nt) o[nt][0] = o[nt][1] = o[nt][2] = o[nt][3] = 0.f;
-  float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
+  for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+    for (int e = 0; e < 2 * NR; ++e) o[nt][e] = 0.f;
+  float m_run[NR], l_run[NR];
+#pragma unroll
+  for (int i = 0; i < NR; ++i) {
+    m_run[i] = -INFINITY;
+    l_run[i] = 0.f;
+  }
 
   uint8_t* my_stage = att_smem + (size_t)warp * STAGES * STAGE_BYTES;
   const int* bt = a.block_tables + (size_t)b * a.max_blocks;
@@ -288,22 +313,22 @@ paged_attention_kernel(const AttnArgs a, int G /*q heads per kv head*/) {
   pdl_wait();
   ATT_STAMP(1);
   // Q fragments (A operand), straight from global memory
-  uint32_t qf[KS][4];
+  uint32_t qf[KS][2 * NR];
   if constexpr (MODE == 0) {
 #pragma unroll
     for (int ks = 0; ks < KS; ++ks) {
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
+      for (int i = 0; i < NR; ++i) {
         const __nv_bfloat16* qp = a.q + ((size_t)(q0 + qtok[i]) * a.nq + kvh * G + hg[i]) * HD + ks * 16 + 2 * t4;
         qf[ks][i] = rvalid[i] ? *reinterpret_cast<const uint32_t*>(qp) : 0u;
-        qf[ks][i + 2] = rvalid[i] ? *reinterpret_cast<const uint32_t*>(qp + 8) : 0u;
+        qf[ks][NR + i] = rvalid[i] ? *reinterpret_cast<const uint32_t*>(qp + 8) : 0u;
       }
     }
   } else {
 #pragma unroll
     for (int gi = 0; gi < NG; ++gi) {
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
+      for (int i = 0; i < NR; ++i) {
         const uint32_t* qp =
             reinterpret_cast<const uint32_t*>(a.q + ((size_t)(q0 + qtok[i]) * a.nq + kvh * G + hg[i]) * HD + gi * 32 + 8 * t4);
         uint32_t w[4];  // channels (0, 1) (2, 3) (4, 5) (6, 7) of this lane's eight
@@ -312,9 +337,9 @@ paged_attention_kernel(const AttnArgs a, int G /*q heads per kv head*/) {
         constexpr int X = 0, Y = MODE == 3 ? 2 : 1, Z = MODE == 3 ? 1 : 2, W = 3;
         // q4: (0, 4) (1, 5) | (2, 6) (3, 7), the nibbles that lie 16 bits apart; q8: (0, 2) (1, 3) | (4, 6) (5, 7)
         qf[2 * gi][i] = att_prmt<0x5410>(w[X], w[Y]);
-        qf[2 * gi][i + 2] = att_prmt<0x7632>(w[X], w[Y]);
+        qf[2 * gi][NR + i] = att_prmt<0x7632>(w[X], w[Y]);
         qf[2 * gi + 1][i] = att_prmt<0x5410>(w[Z], w[W]);
-        qf[2 * gi + 1][i + 2] = att_prmt<0x7632>(w[Z], w[W]);
+        qf[2 * gi + 1][NR + i] = att_prmt<0x7632>(w[Z], w[W]);
       }
     }
   }
@@ -347,7 +372,9 @@ paged_attention_kernel(const AttnArgs a, int G /*q heads per kv head*/) {
     const int page = page_lo + first + it * stride;
 
     // S = Q K^T for 16 tokens: 2 n-tiles
-    float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+    float s[2][2 * NR];
+#pragma unroll
+    for (int e = 0; e < 2 * NR; ++e) s[0][e] = s[1][e] = 0.f;
     if constexpr (MODE == 0) {
       const int mi = lane >> 3, r = lane & 7;
       const uint32_t addr0 = smem_u32(st) + ((mi >> 1) * 8 + r) * ROWB + (mi & 1) * 16;
@@ -355,8 +382,8 @@ paged_attention_kernel(const AttnArgs a, int G /*q heads per kv head*/) {
       for (int ks = 0; ks < KS; ++ks) {
         uint32_t b0, b1, b2, b3;
         ldmatrix_x4(addr0 + ks * 32, b0, b1, b2, b3);
-        mma_bf16_16816(s[0], qf[ks], b0, b1);
-        mma_bf16_16816(s[1], qf[ks], b2, b3);
+        att_mma<NR>(s[0], qf[ks], b0, b1);
+        att_mma<NR>(s[1], qf[ks], b2, b3);
       }
     } else {
       const float* sc = reinterpret_cast<const float*>(st + 32 * ROWB) + 2 * t4 * NG;  // scales of keys 2 t4, 2 t4 + 1 (+ 8)
@@ -377,22 +404,25 @@ paged_attention_kernel(const AttnArgs a, int G /*q heads per kv head*/) {
             b[2] = att_q8_pair(w.y, att_prmt<0xAA88>(w.y, 0u));
             b[3] = att_q8_pair(w.y >> 8, att_prmt<0xBB99>(w.y, 0u));
           }
-          float part[4] = {0.f, 0.f, 0.f, 0.f};
-          mma_bf16_16816(part, qf[2 * gi], b[0], b[1]);
-          mma_bf16_16816(part, qf[2 * gi + 1], b[2], b[3]);
+          float part[2 * NR];
+#pragma unroll
+          for (int e = 0; e < 2 * NR; ++e) part[e] = 0.f;
+          att_mma<NR>(part, qf[2 * gi], b[0], b[1]);
+          att_mma<NR>(part, qf[2 * gi + 1], b[2], b[3]);
           const float k0 = sc[nt * 8 * NG + gi], k1 = sc[(nt * 8 + 1) * NG + gi];
-          s[nt][0] += part[0] * k0;
-          s[nt][1] += part[1] * k1;
-          s[nt][2] += part[2] * k0;
-          s[nt][3] += part[3] * k1;
+#pragma unroll
+          for (int i = 0; i < NR; ++i) {
+            s[nt][2 * i] += part[2 * i] * k0;
+            s[nt][2 * i + 1] += part[2 * i + 1] * k1;
+          }
         }
       }
     }
     // scale, mask, online softmax (rows g and g+8; a quad holds one row's 16 scores)
     const int key0 = page * ATT_PAGE;
-    float p[2][4];
+    float p[2][2 * NR];
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < NR; ++i) {
       float mx = -INFINITY;
 #pragma unroll
       for (int nt = 0; nt < 2; ++nt) {
@@ -433,19 +463,20 @@ paged_attention_kernel(const AttnArgs a, int G /*q heads per kv head*/) {
     }
     // O += P V : P (16x16) as A fragment, V page as B via transposing ldmatrix
     if constexpr (MODE == 0) {
-      uint32_t pf[4];
-      pf[0] = pack_bf16x2(p[0][0], p[0][1]);
-      pf[1] = pack_bf16x2(p[0][2], p[0][3]);
-      pf[2] = pack_bf16x2(p[1][0], p[1][1]);
-      pf[3] = pack_bf16x2(p[1][2], p[1][3]);
+      uint32_t pf[2 * NR];
+#pragma unroll
+      for (int i = 0; i < NR; ++i) {
+        pf[i] = pack_bf16x2(p[0][2 * i], p[0][2 * i + 1]);
+        pf[NR + i] = pack_bf16x2(p[1][2 * i], p[1][2 * i + 1]);
+      }
       const int mi = lane >> 3, r = lane & 7;
       const uint32_t addr0 = smem_u32(st) + 16 * ROWB + ((mi & 1) * 8 + r) * ROWB + (mi >> 1) * 16;
 #pragma unroll
       for (int nt = 0; nt < NT; nt += 2) {
         uint32_t b0, b1, b2, b3;
         ldmatrix_x4_trans(addr0 + nt * 16, b0, b1, b2, b3);
-        mma_bf16_16816(o[nt], pf, b0, b1);
-        mma_bf16_16816(o[nt + 1], pf, b2, b3);
+        att_mma<NR>(o[nt], pf, b0, b1);
+        att_mma<NR>(o[nt + 1], pf, b2, b3);
       }
     } else {
       // this lane's tokens are 2 t4, 2 t4 + 1 and those 8 further; column n of tile 4 gi + j is channel 32 gi + 4 n + j
@@ -453,12 +484,12 @@ paged_attention_kernel(const AttnArgs a, int G /*q heads per kv head*/) {
       const uint8_t* row = st + (16 + 2 * t4) * ROWB;
 #pragma unroll
       for (int gi = 0; gi < NG; ++gi) {
-        uint32_t pf[4], b[2][4];
+        uint32_t pf[2 * NR], b[2][4];
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt) {
           const float v0 = sc[nt * 8 * NG + gi], v1 = sc[(nt * 8 + 1) * NG + gi];
-          pf[2 * nt] = pack_bf16x2(p[nt][0] * v0, p[nt][1] * v1);
-          pf[2 * nt + 1] = pack_bf16x2(p[nt][2] * v0, p[nt][3] * v1);
+#pragma unroll
+          for (int i = 0; i < NR; ++i) pf[NR * nt + i] = pack_bf16x2(p[nt][2 * i] * v0, p[nt][2 * i + 1] * v1);
           const uint8_t* r0 = row + nt * 8 * ROWB;
           if constexpr (MODE == 3) {
             const uint32_t w = (uint32_t)*reinterpret_cast<const uint16_t*>(r0 + gi * 16 + 2 * g) |
@@ -475,7 +506,7 @@ paged_attention_kernel(const AttnArgs a, int G /*q heads per kv head*/) {
           }
         }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) mma_bf16_16816(o[4 * gi + j], pf, b[0][j], b[1][j]);
+        for (int j = 0; j < 4; ++j) att_mma<NR>(o[4 * gi + j], pf, b[0][j], b[1][j]);
       }
     }
     __syncwarp();
@@ -493,7 +524,7 @@ paged_attention_kernel(const AttnArgs a, int G /*q heads per kv head*/) {
 #pragma unroll
   for (int nt = 0; nt < NT; ++nt) {
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < NR; ++i) {
       if (rvalid[i]) {
         float* row = mo + ((size_t)warp * 16 + g + 8 * i) * HD;
         if constexpr (MODE == 0) {
@@ -509,7 +540,7 @@ paged_attention_kernel(const AttnArgs a, int G /*q heads per kv head*/) {
   }
   if (t4 == 0) {
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < NR; ++i) {
       if (rvalid[i]) {
         mml[(warp * 16 + g + 8 * i) * 2] = m_run[i];
         mml[(warp * 16 + g + 8 * i) * 2 + 1] = l_run[i];

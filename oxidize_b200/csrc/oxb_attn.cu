@@ -14,12 +14,12 @@ OXB_API int oxb_attn_ws_floats(int B, int nkv, int max_mtiles, int n_cta_splits,
   return 0;
 }
 
-template <int HD, int MODE = 0>
-static int attn_launch(const AttnArgs& a, int B, int G, cudaStream_t stream) {
+template <int HD, int MODE, int NR>
+static int attn_launch_rows(const AttnArgs& a, int B, int G, cudaStream_t stream) {
   constexpr int smem = AttPage<HD, MODE>::SMEM;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(paged_attention_kernel<HD, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(paged_attention_kernel<HD, MODE, NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
@@ -27,9 +27,17 @@ static int attn_launch(const AttnArgs& a, int B, int G, cudaStream_t stream) {
   // (The KV splits of a row tile stay independent CTAs and the last one to finish merges: inside a thread-block
   // cluster every CTA would wait for the slowest split.)
   if (a.n_cta_splits > 1 && (a.ws_o == nullptr || a.ws_ml == nullptr || a.counters == nullptr)) return (int)cudaErrorInvalidValue;
-  oxb_launch(paged_attention_kernel<HD, MODE>, grid, dim3(ATT_WARPS * 32), (size_t)smem, stream, a, G);
+  oxb_launch(paged_attention_kernel<HD, MODE, NR>, grid, dim3(ATT_WARPS * 32), (size_t)smem, stream, a, G);
   OXB_CHECK_LAUNCH();
   return 0;
+}
+
+template <int HD, int MODE = 0>
+static int attn_launch(const AttnArgs& a, int B, int G, int max_query_len, cudaStream_t stream) {
+  if constexpr (HD == 64 || HD == 128) {
+    if (max_query_len * G <= 8) return attn_launch_rows<HD, MODE, 1>(a, B, G, stream);
+  }
+  return attn_launch_rows<HD, MODE, 2>(a, B, G, stream);
 }
 
 OXB_API int oxb_paged_attention(const void* q, void* out, const void* kv_data, const float* kv_scales,
@@ -70,17 +78,17 @@ OXB_API int oxb_paged_attention(const void* q, void* out, const void* kv_data, c
   a.num_blocks = num_blocks;
   a.max_rows = max_rows;
   a.trace = g_oxb_attn_trace;
-  if (kv_mode == 2 && hd == 128) return attn_launch<128, 2>(a, B, G, stream);
-  if (kv_mode == 2 && hd == 64) return attn_launch<64, 2>(a, B, G, stream);
-  if (kv_mode == 3 && hd == 128) return attn_launch<128, 3>(a, B, G, stream);
-  if (kv_mode == 3 && hd == 64) return attn_launch<64, 3>(a, B, G, stream);
-  if (hd == 128) return attn_launch<128>(a, B, G, stream);
-  if (hd == 64) return attn_launch<64>(a, B, G, stream);
+  if (kv_mode == 2 && hd == 128) return attn_launch<128, 2>(a, B, G, max_query_len, stream);
+  if (kv_mode == 2 && hd == 64) return attn_launch<64, 2>(a, B, G, max_query_len, stream);
+  if (kv_mode == 3 && hd == 128) return attn_launch<128, 3>(a, B, G, max_query_len, stream);
+  if (kv_mode == 3 && hd == 64) return attn_launch<64, 3>(a, B, G, max_query_len, stream);
+  if (hd == 128) return attn_launch<128>(a, B, G, max_query_len, stream);
+  if (hd == 64) return attn_launch<64>(a, B, G, max_query_len, stream);
   if (kv_mode != 0) return (int)cudaErrorInvalidValue;
-  if (hd == 32) return attn_launch<32>(a, B, G, stream);
-  if (hd == 96) return attn_launch<96>(a, B, G, stream);
-  if (hd == 192) return attn_launch<192>(a, B, G, stream);
-  if (hd == 256) return attn_launch<256>(a, B, G, stream);
+  if (hd == 32) return attn_launch<32>(a, B, G, max_query_len, stream);
+  if (hd == 96) return attn_launch<96>(a, B, G, max_query_len, stream);
+  if (hd == 192) return attn_launch<192>(a, B, G, max_query_len, stream);
+  if (hd == 256) return attn_launch<256>(a, B, G, max_query_len, stream);
   return (int)cudaErrorInvalidValue;
 }
 
