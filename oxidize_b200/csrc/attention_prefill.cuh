@@ -46,7 +46,7 @@ __device__ __forceinline__ int prefill_page_base(const int* query_start, const i
   return __reduce_add_sync(0xffffffffu, n);
 }
 
-// f16 / q8 / q4 pages of the long sequences as bf16 pages, one CTA per page: out [pages, nkv, K | V, 16, HD].
+// f16 / q8 / q4 pages of the long sequences as bf16 pages, a CTA for every page and head: out [pages, nkv, K | V, 16, HD].
 template <int HD, int MODE>
 static __global__ void __launch_bounds__(256)
 prefill_pages_kernel(const uint8_t* __restrict__ cache, const float* __restrict__ scales, const int* __restrict__ query_start,
@@ -65,9 +65,9 @@ prefill_pages_kernel(const uint8_t* __restrict__ cache, const float* __restrict_
     if (threadIdx.x == 0) oxb_report(OXB_BAD_BLOCK_ID, blk);
     blk = 0;
   }
-  const int rows = nkv * 2 * ATT_PAGE;
-  const size_t row0 = (size_t)blk * rows;
-  __nv_bfloat16* o = out + (size_t)dst_page * rows * HD;
+  const int rows = 2 * ATT_PAGE;  // of this head
+  const size_t row0 = ((size_t)blk * nkv + blockIdx.z) * rows;
+  __nv_bfloat16* o = out + ((size_t)dst_page * nkv + blockIdx.z) * rows * HD;
   for (int c = threadIdx.x; c < rows * (HD / 8); c += 256) {  // 8 values
     const int row = c / (HD / 8), col = (c % (HD / 8)) * 8;
     float v[8];

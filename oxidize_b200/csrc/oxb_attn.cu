@@ -99,7 +99,7 @@ static int prefill_convert(int mode, const void* kv_data, const float* kv_scales
                            const int* query_start, int B, int max_blocks, int num_blocks, int nkv, int max_pages, int cap_pages,
                            int window, int min_rows, __nv_bfloat16* pages, cudaStream_t stream) {
   const uint8_t* src = reinterpret_cast<const uint8_t*>(kv_data);
-  const dim3 grid(max_pages, B), block(256);
+  const dim3 grid(max_pages, B, nkv), block(256);
   auto go = [&](auto kernel) {
     return oxb_launch(kernel, grid, block, 0, stream, src, kv_scales, query_start, seq_lens, block_tables, max_blocks, num_blocks, nkv,
                       window, min_rows, cap_pages, pages);

@@ -2,6 +2,7 @@
 import pytest
 import torch
 
+from oxidize_b200 import ops
 from oxidize_b200.engine.kv_pool import KVCache, KVCacheSpec
 from oxidize_b200.models.transformer import BatchMeta
 from oxidize_b200.models.weights import qtensor_from_dense
@@ -96,6 +97,39 @@ def test_quantized_pages_in_fragments(C, kvd, hd, nq, nkv, lens):
         _check_status(C)
         # codes are exact; the output and the scaled probabilities are rounded to bf16
         assert _off(got, want) < 4e-3
+
+
+@pytest.mark.parametrize("kvd", ["bf16", "f16", "q8", "q4"])
+@pytest.mark.parametrize("hd,rot,pairing,norm", [(64, 64, "split_half", True), (64, 32, "adjacent", False), (128, 128, "adjacent", True),
+                                                 (128, 96, "split_half", False), (256, 64, "split_half", True), (256, 256, "adjacent", False),
+                                                 (128, 20, "split_half", True), (96, 96, "split_half", False)])
+def test_rotation_and_cache_rows_of_a_warp_to_a_head(C, kvd, hd, rot, pairing, norm):
+    """Widths and rotations that a warp per head takes (the last two: that it does not), a token count that fills no CTA."""
+    from types import SimpleNamespace
+
+    gen = torch.Generator().manual_seed(hd + rot)
+    T, nq, nkv = 11, 3, 2
+    qkv = torch.randn(T, (nq + 2 * nkv) * hd, generator=gen).bfloat16()
+    pos = torch.tensor([0, 1, 2, 40, 41, 7, 100, 3000, 5, 6, 9], dtype=torch.int32)
+    slots = torch.tensor([0, 1, 2, 56, 57, 23, -1, 90, 21, 22, 127], dtype=torch.int32)
+    norms = [torch.rand(hd, generator=gen) + 0.5 if norm else None for _ in range(2)]
+    caches, queries = [], []
+    for dev in ("cpu", "cuda"):
+        kv = KVCache(KVCacheSpec(1, nkv, hd, 16, kvd), 8, torch.device(dev))
+        rope = SimpleNamespace(inv_freq=ref.rope_inv_freq(rot, 10000.0, None, device=dev), pairing=pairing, mscale=1.0, n_heads=nq,
+                               n_kv_heads=nkv, head_dim=hd, max_pos=0)
+        x = qkv.float() if dev == "cpu" else qkv.cuda()
+        queries.append(ops.qk_rope_kv_write(x, pos.to(dev), slots.to(dev), kv, 0, rope,
+                                            *[None if n is None else n.to(dev) for n in norms], 1e-6))
+        caches.append(kv)
+    _check_status(C)
+    assert _off(queries[1], queries[0]) < 3e-3  # rounded to bf16
+    back = KVCache(caches[0].spec, 8, torch.device("cpu"))
+    back.data, back.scales = [d.cpu() for d in caches[1].data], [None if s is None else s.cpu() for s in caches[1].scales]
+    table = torch.arange(8, dtype=torch.int32)
+    for got, want in zip(ref.kv_gather(back, 0, table, 128), ref.kv_gather(caches[0], 0, table, 128)):
+        # (quantized: a code may fall to the other side where a value lies between two; one step of 32 values' largest)
+        assert _off(got, want) < {"bf16": 3e-3, "f16": 1e-3, "q8": 2e-3, "q4": 3e-2}[kvd]
 
 
 # ------------------------------------------------------------------------------------------- packed GEMM
