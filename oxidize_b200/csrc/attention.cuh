@@ -1,4 +1,5 @@
-// Paged GQA flash attention for decode, speculative verify and chunked prefill in one kernel.
+// Paged GQA flash attention for decode, speculative verify and short portions of prompts in one kernel (long portions of heads of 64
+// and 128: attention_prefill.cuh).
 //
 // Work decomposition: a CTA owns (sequence, kv head, 16-row query tile, CTA split); a "row" is a
 // (query token, head-in-group) pair, so the 8 query heads that share one KV head in the 70B / 8B

@@ -405,7 +405,7 @@ struct GroupArgs {
 
 // Most token tiles that `rows` rows in `groups` groups of at most max_rows rows can make
 inline long long gathered_tiles(long long rows, int groups, int max_rows, int tn) {
-  const long long by_rows = rows / tn + groups, by_group = (long long)groups * ((max_rows + tn - 1) / tn);
+  const long long by_rows = rows / tn + (rows < groups ? rows : groups), by_group = (long long)groups * ((max_rows + tn - 1) / tn);
   return by_rows < by_group ? by_rows : by_group;
 }
 
@@ -1145,7 +1145,8 @@ inline GemmPlan gemm_plan(int T, int N, int K, int splits_hint, int sm_count, in
     const int tiles = p.n_tiles * p.t_tiles;
     const int resident = sm_count * (p.tn <= 64 ? 2 : 1);
     // Tiles wider than 64 tokens hold one CTA per SM, and their partials are large: split only
-    // within one wave.  Nothing is split once the tiles alone fill the SMs.
+    // within one wave.  Nothing is split once the tiles alone fill the SMs (groups: four times, as their tiles are many
+    // at once and a split evens out the last wave: 8 experts of 4096 x 14336, 64 tokens, 256 tiles).
     const int wave_cap = p.tn <= 64 ? (1 << 30) : sm_count;
     int capacity = max_ctas > 0 ? max_ctas : (cluster_ok ? wave_cap : resident);
     if (capacity > wave_cap) capacity = wave_cap;
@@ -1154,7 +1155,7 @@ inline GemmPlan gemm_plan(int T, int N, int K, int splits_hint, int sm_count, in
     long long best_cost = -1;
     splits = 1;
     const int s_max = p.tn <= 64 ? 16 : 4;  // wide tiles have large partials: a deep split costs more than it streams
-    for (int s = 1; s <= s_max && s <= max_by_k && (long long)tiles * s <= capacity && (s == 1 || tiles * groups < sm_count); ++s) {
+    for (int s = 1; s <= s_max && s <= max_by_k && (long long)tiles * s <= capacity && (s == 1 || (long long)tiles * groups < (groups > 1 ? 4 : 1) * sm_count); ++s) {
       const int per_cta = (kb_total + s - 1) / s;
       long long cost;
       if (packed) {

@@ -40,12 +40,11 @@ static int attn_launch(const AttnArgs& a, int B, int G, int max_query_len, cudaS
   return attn_launch_rows<HD, MODE, 2>(a, B, G, stream);
 }
 
-OXB_API int oxb_paged_attention(const void* q, void* out, const void* kv_data, const float* kv_scales,
-                                const int* block_tables, const int* seq_lens, const int* query_start, int B,
-                                int max_blocks, int nq, int nkv, int hd, int kv_mode, int max_query_len,
-                                int n_cta_splits, int window, float scale, float softcap, const float* sink, int ld_out,
-                                float out_scale, float* ws_o, float* ws_ml, int* counters, int num_blocks,
-                                const void* gate, int ld_gate, int gate_per_value, int max_rows, cudaStream_t stream) {
+static int paged_attention(const void* q, void* out, const void* kv_data, const float* kv_scales, const int* block_tables,
+                           const int* seq_lens, const int* query_start, int B, int max_blocks, int nq, int nkv, int hd, int kv_mode,
+                           int max_query_len, int n_cta_splits, int window, float scale, float softcap, const float* sink, int ld_out,
+                           float out_scale, float* ws_o, float* ws_ml, int* counters, int num_blocks, const void* gate, int ld_gate,
+                           int gate_per_value, int max_rows, cudaStream_t stream) {
   if (B <= 0) return 0;
   if (nq % nkv != 0 || (gate != nullptr && gate_per_value && (ld_gate % 2 != 0 || (reinterpret_cast<uintptr_t>(gate) & 3) != 0)))
     return (int)cudaErrorInvalidValue;
@@ -90,6 +89,29 @@ OXB_API int oxb_paged_attention(const void* q, void* out, const void* kv_data, c
   if (hd == 192) return attn_launch<192>(a, B, G, max_query_len, stream);
   if (hd == 256) return attn_launch<256>(a, B, G, max_query_len, stream);
   return (int)cudaErrorInvalidValue;
+}
+
+OXB_API int oxb_paged_attention(const void* q, void* out, const void* kv_data, const float* kv_scales,
+                                const int* block_tables, const int* seq_lens, const int* query_start, int B,
+                                int max_blocks, int nq, int nkv, int hd, int kv_mode, int max_query_len,
+                                int n_cta_splits, int window, float scale, float softcap, const float* sink, int ld_out,
+                                float out_scale, float* ws_o, float* ws_ml, int* counters, int num_blocks,
+                                const void* gate, int ld_gate, int gate_per_value, cudaStream_t stream) {
+  return paged_attention(q, out, kv_data, kv_scales, block_tables, seq_lens, query_start, B, max_blocks, nq, nkv, hd, kv_mode,
+                         max_query_len, n_cta_splits, window, scale, softcap, sink, ld_out, out_scale, ws_o, ws_ml, counters,
+                         num_blocks, gate, ld_gate, gate_per_value, 0, stream);
+}
+
+// The same for the sequences that feed fewer than max_rows rows (max_query_len: the most of those); the others are left alone.
+OXB_API int oxb_paged_attention_short(const void* q, void* out, const void* kv_data, const float* kv_scales,
+                                      const int* block_tables, const int* seq_lens, const int* query_start, int B,
+                                      int max_blocks, int nq, int nkv, int hd, int kv_mode, int max_query_len,
+                                      int n_cta_splits, int window, float scale, float softcap, const float* sink, int ld_out,
+                                      float out_scale, float* ws_o, float* ws_ml, int* counters, int num_blocks,
+                                      const void* gate, int ld_gate, int gate_per_value, int max_rows, cudaStream_t stream) {
+  return paged_attention(q, out, kv_data, kv_scales, block_tables, seq_lens, query_start, B, max_blocks, nq, nkv, hd, kv_mode,
+                         max_query_len, n_cta_splits, window, scale, softcap, sink, ld_out, out_scale, ws_o, ws_ml, counters,
+                         num_blocks, gate, ld_gate, gate_per_value, max_rows, stream);
 }
 
 

@@ -423,8 +423,10 @@ OXB_API int oxb_gemm_grouped_rows(const void* X, int rows_cap, const void* W, in
   const long long avg = ((long long)rows_cap + groups - 1) / groups;
   int rows = 2 * avg < max_rows ? (int)(2 * avg) : max_rows;
   if (packed && avg <= 96 && rows > 128) rows = 128;  // (most groups fit a tile of 128: one of 256 would only be emptier)
-  GemmPlan p = gemm_plan(rows, N, K, 0, sm_count(), 1, 0, packed, groups);
-  if (p.splits > 1 && !p.cluster) p = gemm_plan(rows, N, K, 1, sm_count(), 1, 0, packed, groups);
+  // (no more groups than rows have any: one token of 8 experts leaves SMs idle that splits along K fill)
+  const int active = rows_cap < groups ? rows_cap : groups;
+  GemmPlan p = gemm_plan(rows, N, K, 0, sm_count(), 1, 0, packed, active);
+  if (p.splits > 1 && !p.cluster) p = gemm_plan(rows, N, K, 1, sm_count(), 1, 0, packed, active);
   p.t_tiles = (int)gathered_tiles(rows_cap, groups, max_rows, p.tn);
   CUtensorMap tmW, tmX;
   int e = oxb_make_tmap_2d(&tmX, X, (uint64_t)rows_cap, K, (uint64_t)K * 2, p.tn, GEMM_BK, 2);

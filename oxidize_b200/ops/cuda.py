@@ -122,7 +122,7 @@ def _declare(L) -> None:
     L.oxb_qk_rope_kvwrite.argtypes = [vp, vp, vp, vp, i32, i32, i32, vp, vp, f32, i32, i32, i32, i32, vp, vp, vp, i32,
                                       i32, i32, vp]
     L.oxb_argmax.argtypes = [vp, i32, i32, i32, i32, vp, vp, i32, vp]
-    L.oxb_paged_attention.argtypes = [vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, f32, f32,
+    L.oxb_paged_attention_short.argtypes = [vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, f32, f32,
                                       vp, i32, f32, vp, vp, vp, i32, vp, i32, i32, i32, vp]
     L.oxb_paged_prefill.argtypes = [vp] * 7 + [i32] * 10 + [f32, vp, i32, f32, i32, vp, i32, i32, vp, i32, i32, vp]
     L.oxb_paged_prefill_supported.argtypes = [i32] * 3
@@ -583,13 +583,13 @@ def paged_attention(q, kv, layer, meta, scale, sliding_window=0, splits: Optiona
         tasks = B * nkv * mtiles * splits
         ws_o, ws_ml = scratch(q.device).attn(tasks * 16 * hd, tasks * 32)
         cnt = scratch(q.device).attn_counters
-    _check(lib().oxb_paged_attention(q.data_ptr(), out.data_ptr(), kv.data[layer].data_ptr(), _p(kv.scales[layer]),
+    _check(lib().oxb_paged_attention_short(q.data_ptr(), out.data_ptr(), kv.data[layer].data_ptr(), _p(kv.scales[layer]),
                                      meta.block_tables.data_ptr(), meta.seq_lens.data_ptr(), meta.query_start.data_ptr(),
                                      B, meta.block_tables.stride(0), nq, nkv, hd, KV_MODE[kv.dtype_name],
                                      query_len, splits, sliding_window, scale, float(softcap), _p(sink),
                                      out.stride(0), out_scale, _p(ws_o), _p(ws_ml), _p(cnt), kv.num_blocks, _p(gate),
                                      0 if gate is None else gate.stride(0), int(gate_per_value), short_below, _stream()),
-           "oxb_paged_attention")
+           "oxb_paged_attention_short")
     return out
 
 
