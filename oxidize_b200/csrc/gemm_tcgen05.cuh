@@ -1145,8 +1145,9 @@ inline GemmPlan gemm_plan(int T, int N, int K, int splits_hint, int sm_count, in
     const int tiles = p.n_tiles * p.t_tiles;
     const int resident = sm_count * (p.tn <= 64 ? 2 : 1);
     // Tiles wider than 64 tokens hold one CTA per SM, and their partials are large: split only
-    // within one wave.  Nothing is split once the tiles alone fill the SMs (groups: four times, as their tiles are many
-    // at once and a split evens out the last wave: 8 experts of 4096 x 14336, 64 tokens, 256 tiles).
+    // within one wave.  Nothing is split once the tiles alone fill the SMs; in groups whose tiles are small and rows long, four
+    // times, as a split evens out the last wave (8 experts of 4096 x 14336, bf16, 64 tokens, 256 tiles: 196 us unsplit, 177 split; but
+    // 200 tokens in tiles of 256 169 and 214, and rows of 4096, 28672 of them, one token 86 and 94).
     const int wave_cap = p.tn <= 64 ? (1 << 30) : sm_count;
     int capacity = max_ctas > 0 ? max_ctas : (cluster_ok ? wave_cap : resident);
     if (capacity > wave_cap) capacity = wave_cap;
@@ -1155,7 +1156,7 @@ inline GemmPlan gemm_plan(int T, int N, int K, int splits_hint, int sm_count, in
     long long best_cost = -1;
     splits = 1;
     const int s_max = p.tn <= 64 ? 16 : 4;  // wide tiles have large partials: a deep split costs more than it streams
-    for (int s = 1; s <= s_max && s <= max_by_k && (long long)tiles * s <= capacity && (s == 1 || (long long)tiles * groups < (groups > 1 ? 4 : 1) * sm_count); ++s) {
+    for (int s = 1; s <= s_max && s <= max_by_k && (long long)tiles * s <= capacity && (s == 1 || (long long)tiles * groups < (groups > 1 && p.tn <= 64 && kb_total >= 128 ? 4 : 1) * sm_count); ++s) {
       const int per_cta = (kb_total + s - 1) / s;
       long long cost;
       if (packed) {
@@ -1183,6 +1184,29 @@ inline GemmPlan gemm_plan(int T, int N, int K, int splits_hint, int sm_count, in
   p.ws_bytes = scratch ? (size_t)p.n_tiles * p.t_tiles * splits * p.tn * GEMM_BM * sizeof(float) : 0;
   p.n_counters = scratch ? 2 * p.n_tiles * p.t_tiles : 0;
   return p;
+}
+
+// Plan of a gathered launch: `rows` rows at most in all groups together, `expected` of them on average (fewer where the groups are the
+// experts of one rank among several).
+inline GemmPlan gathered_plan(int rows, int expected, int groups, int max_rows, int N, int K, int sm_count, bool packed) {
+  // The token tile follows the rows that a group has on average (twice that, so that most groups fit into one tile), not
+  // the most that one could have: tiles only for the routed rows are run, so a fuller group just takes more of them.
+  // (128 experts of 1536 x 2048, 640 rows: 385 us with tiles of 128 rows for the 80 that one expert could have had, 136 us,
+  // 5.9 TB/s, with tiles of 16.)
+  const long long avg = ((long long)rows + groups - 1) / groups;
+  int most = 2 * avg < max_rows ? (int)(2 * avg) : max_rows;
+  // Up to 112 rows on average most groups fit a tile of 128, and one of 256 would only be emptier (400 tokens, 2 of 8 experts each,
+  // us with tiles of 256 and of 128: 28672 x 4096 Q4_K 408 and 296, bf16 450 and 360; 4096 x 14336 195 and 131, 268 and 174).
+  // Packed weights go by the rows that are expected: among all rows of the step a rank's experts would look fuller than they
+  // are (2 of 8 experts, 200 tokens: 129 and 91).  For bf16 weights, which are read once in either tile, the most rows count.
+  if ((packed ? ((long long)expected + groups - 1) / groups : avg) <= 112 && most > 128) most = 128;
+  // A packed tile costs its decoding whether 16 tokens or 32 use it: the tokens of a group that is fuller than the others then
+  // take half as many (128 experts of 2048 x 768, Q4_K, 128 tokens, most to 8 of them: 157 us and 132; spread evenly 134 and 130).
+  if (packed && most < 32) most = max_rows < 32 ? max_rows : 32;
+  // (no more groups than rows have any: one token of 8 experts leaves SMs idle that splits along K fill)
+  const int active = rows < groups ? rows : groups;
+  const GemmPlan p = gemm_plan(most, N, K, 0, sm_count, 1, 0, packed, active);
+  return p.splits > 1 && !p.cluster ? gemm_plan(most, N, K, 1, sm_count, 1, 0, packed, active) : p;
 }
 
 // Largest cluster the kernel instance can be launched with: 16 where the device accepts the

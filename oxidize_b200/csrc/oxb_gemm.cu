@@ -405,29 +405,35 @@ OXB_API int oxb_gemm_batched(const void* X, const void* W, void* Y, long long y_
   }
 }
 
+// The plan of oxb_gemm_grouped_rows: token tile, weight tiles, token tiles at most, splits
+OXB_API int oxb_gemm_grouped_rows_plan(int rows_cap, int qtype, int groups, int max_rows, int expected_rows, int N, int K, int* out4) {
+  if (rows_cap <= 0 || max_rows <= 0 || N <= 0 || K <= 0 || groups <= 0) return (int)cudaErrorInvalidValue;
+  if (expected_rows <= 0 || expected_rows > rows_cap) expected_rows = rows_cap;
+  const GemmPlan p = gathered_plan(rows_cap, expected_rows, groups, max_rows, N, K, sm_count(), qtype != QT_BF16);
+  out4[0] = p.tn;
+  out4[1] = p.n_tiles;
+  out4[2] = (int)gathered_tiles(rows_cap, groups, max_rows, p.tn);
+  out4[3] = p.splits;
+  return 0;
+}
+
 // Grouped GEMM over token-gathered groups (mixture-of-experts dispatch): group g multiplies the activation rows
 // [row_offsets[g], row_offsets[g+1]) of X ([rows_cap, K], gathered expert by expert) with its own weights
 // W_g ([N, K] at rows g*N of the stacked matrix) and writes the same rows of Y ([rows_cap, ldY]).  row_offsets is a
 // device array of groups + 1 ints written by the upstream kernel; max_rows bounds the rows of any one group (with rows_cap
-// it bounds the grid).
+// it bounds the grid); expected_rows: how many all groups together are expected to have (0: rows_cap, as where the groups
+// are all experts; a rank's share of it where they are one rank's).
 OXB_API int oxb_gemm_grouped_rows(const void* X, int rows_cap, const void* W, int qtype, size_t row_bytes, void* Y,
-                                  const int* row_offsets, int groups, int max_rows, int N, int K, int ldY,
+                                  const int* row_offsets, int groups, int max_rows, int expected_rows, int N, int K, int ldY,
                                   int epi, cudaStream_t stream) {
   if (rows_cap <= 0 || max_rows <= 0 || N <= 0 || K <= 0 || groups <= 0) return 0;
   if (K % 64 != 0 || row_offsets == nullptr || (epi != EPI_STORE && epi != EPI_RELU2)) return (int)cudaErrorInvalidValue;
   const bool packed = qtype != QT_BF16;
-  // The token tile follows the rows that a group has on average (twice that, so that most groups fit into one tile), not
-  // the most that one could have: tiles only for the routed rows are run, so a fuller group just takes more of them.
-  // (128 experts of 1536 x 2048, 640 rows: 385 us with tiles of 128 rows for the 80 that one expert could have had, 136 us,
-  // 5.9 TB/s, with tiles of 16.)
-  const long long avg = ((long long)rows_cap + groups - 1) / groups;
-  int rows = 2 * avg < max_rows ? (int)(2 * avg) : max_rows;
-  if (packed && avg <= 96 && rows > 128) rows = 128;  // (most groups fit a tile of 128: one of 256 would only be emptier)
-  // (no more groups than rows have any: one token of 8 experts leaves SMs idle that splits along K fill)
-  const int active = rows_cap < groups ? rows_cap : groups;
-  GemmPlan p = gemm_plan(rows, N, K, 0, sm_count(), 1, 0, packed, active);
-  if (p.splits > 1 && !p.cluster) p = gemm_plan(rows, N, K, 1, sm_count(), 1, 0, packed, active);
-  p.t_tiles = (int)gathered_tiles(rows_cap, groups, max_rows, p.tn);
+  if (expected_rows <= 0 || expected_rows > rows_cap) expected_rows = rows_cap;
+  GemmPlan p = gathered_plan(rows_cap, expected_rows, groups, max_rows, N, K, sm_count(), packed);
+  const long long tiles = gathered_tiles(rows_cap, groups, max_rows, p.tn);
+  if (tiles * p.n_tiles > 0x7FFFFFFF) return (int)cudaErrorInvalidValue;
+  p.t_tiles = (int)tiles;
   CUtensorMap tmW, tmX;
   int e = oxb_make_tmap_2d(&tmX, X, (uint64_t)rows_cap, K, (uint64_t)K * 2, p.tn, GEMM_BK, 2);
   if (e) return e;

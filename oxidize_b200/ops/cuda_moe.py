@@ -39,7 +39,7 @@ def _declare(L):
     L.oxb_moe_permute.argtypes = [vp, i32, i32, i32, i32, vp, vp, vp, vp]
     L.oxb_moe_gather.argtypes = [vp, i32, vp, vp, i32, vp, vp]
     L.oxb_silu_mul_rows.argtypes = [vp, vp, vp, i32, i32, vp]
-    L.oxb_gemm_grouped_rows.argtypes = [vp, i32, vp, i32, sz, vp, vp, i32, i32, i32, i32, i32, i32, vp]
+    L.oxb_gemm_grouped_rows.argtypes = [vp, i32, vp, i32, sz, vp, vp, i32, i32, i32, i32, i32, i32, i32, vp]
     u64p = ctypes.POINTER(ctypes.c_uint64)
     L.oxb_moe_combine_gathered.argtypes = [vp, vp, vp, i32, vp, vp, i32, i32, i32, i32, u64p, u64p, vp, i32, i32, i32,
                                            ctypes.c_ulonglong, vp]
@@ -106,9 +106,11 @@ def moe_combine(y: torch.Tensor, scale: torch.Tensor, shared: Optional[torch.Ten
     return out
 
 
-def gemm_grouped_rows(xg: torch.Tensor, w, offsets: torch.Tensor, groups: int, max_rows: int, epi: int = 0) -> torch.Tensor:
+def gemm_grouped_rows(xg: torch.Tensor, w, offsets: torch.Tensor, groups: int, max_rows: int, epi: int = 0,
+                      expected_rows: int = 0) -> torch.Tensor:
     """y[r] = xg[r] @ W_g^T for every gathered row r of group g (rows [offsets[g], offsets[g+1])); [rows_cap, N] bf16.
-    ``epi``: epilogue of the product (0 none, ``EPI_RELU2``)."""
+    ``epi``: epilogue of the product (0 none, ``EPI_RELU2``); ``expected_rows``: how many of the rows are expected to be in
+    use, where that is not all of them (experts of one rank)."""
     L = C.lib()
     _declare(L)
     N = w.shape[0] // groups
@@ -116,7 +118,7 @@ def gemm_grouped_rows(xg: torch.Tensor, w, offsets: torch.Tensor, groups: int, m
     y = torch.empty(xg.shape[0], N, dtype=torch.bfloat16, device=xg.device)
     row_bytes = w.data.stride(0) * w.data.element_size()
     C._check(L.oxb_gemm_grouped_rows(xg.data_ptr(), xg.shape[0], w.data.data_ptr(), C.QTYPE_CODE[w.qtype], row_bytes,
-                                     y.data_ptr(), offsets.data_ptr(), groups, max_rows, N, K, N, epi, C._stream()),
+                                     y.data_ptr(), offsets.data_ptr(), groups, max_rows, expected_rows, N, K, N, epi, C._stream()),
              "oxb_gemm_grouped_rows")
     return y
 
@@ -180,19 +182,20 @@ def moe_layer(x: torch.Tensor, router_logits: torch.Tensor, cfg, router_bias, ex
         ids, wts = moe_route(router_logits, cfg, router_bias)
         offsets, perm, inv = moe_dispatch(ids, experts.first_expert, E)
         n_rows = offsets[E:]
+        expected = -(-T * k * E // cfg.n_experts)  # of the local experts
         x = x.contiguous()
         xg = torch.empty(T * k, x.shape[1], dtype=torch.bfloat16, device=x.device)
         C._check(L.oxb_moe_gather(x.data_ptr(), x.shape[1], perm.data_ptr(), n_rows.data_ptr(), T * k, xg.data_ptr(),
                                   C._stream()), "oxb_moe_gather")
         if relu2:
-            act = gemm_grouped_rows(xg, experts.gate_up_stack, offsets, E, T, EPI_RELU2)  # [T*k, F]
+            act = gemm_grouped_rows(xg, experts.gate_up_stack, offsets, E, T, EPI_RELU2, expected)  # [T*k, F]
         else:
-            h = gemm_grouped_rows(xg, experts.gate_up_stack, offsets, E, T)  # [T*k, 2F]
+            h = gemm_grouped_rows(xg, experts.gate_up_stack, offsets, E, T, expected_rows=expected)  # [T*k, 2F]
             F = h.shape[1] // 2
             act = torch.empty(T * k, F, dtype=torch.bfloat16, device=x.device)
             C._check(L.oxb_silu_mul_rows(h.data_ptr(), act.data_ptr(), n_rows.data_ptr(), T * k, F, C._stream()),
                      "oxb_silu_mul_rows")
-        y = gemm_grouped_rows(act, experts.down_stack, offsets, E, T)  # [T*k, H]
+        y = gemm_grouped_rows(act, experts.down_stack, offsets, E, T, expected_rows=expected)  # [T*k, H]
         if not combine:
             return y, inv, wts
         return moe_combine_gathered(y, inv, wts, shared, T, comm)

@@ -172,3 +172,45 @@ def test_grouped_rows_lists(C, qtype, N, K, rows):
     full = (w.data if qtype == "BF16" else C.dequant_rows(w)).double().view(E, N, K)
     want = torch.cat([x[a:b].double() @ full[e].t() for e, (a, b) in enumerate(zip(off[:-1].tolist(), off[1:].tolist()))])
     assert _off(got[:R], want) < 8e-3
+
+
+def _worst(got, want):
+    """Largest distance of a row and of a column, each over the root mean square row's or column's norm: a lost edge shows."""
+    d, w = (got.double() - want).cpu(), want.cpu()
+    return max(float(d.norm(dim=i).max() / w.norm(dim=i).square().mean().sqrt()) for i in (0, 1))
+
+
+@pytest.mark.parametrize("qtype", ["BF16", "Q4_K"])
+@pytest.mark.parametrize("N,K,rows", [(260, 2624, [300, 130, 0, 257]), (260, 2304, [150] * 5), (300, 2560, [1] * 200 + [40])])
+def test_grouped_rows_wide_tiles(C, qtype, N, K, rows):
+    """Tiles of 256 rows over rows long enough that every ring wraps; groups by the hundred."""
+    from oxidize_b200.ops import cuda_moe
+
+    if qtype == "Q4_K" and K % 256:
+        K = 2560
+    E, R = len(rows), sum(rows)
+    gen = torch.Generator(device="cuda").manual_seed(R)
+    w = qtensor_from_dense((torch.randn(E * N, K, generator=gen, device="cuda") * 0.05).cpu(), qtype, device="cuda")
+    x = torch.randn(R + 9, K, generator=gen, device="cuda").bfloat16()
+    off = torch.tensor([sum(rows[:i]) for i in range(E + 1)], dtype=torch.int32, device="cuda")
+    got = cuda_moe.gemm_grouped_rows(x, w, off, E, max(rows))
+    _check_status(C)
+    full = (w.data if qtype == "BF16" else C.dequant_rows(w)).double().view(E, N, K)
+    want = torch.cat([x[a:b].double() @ full[e].t() for e, (a, b) in enumerate(zip(off[:-1].tolist(), off[1:].tolist()))])
+    assert _off(got[:R], want) < 8e-3  # (as test_grouped_rows_lists)
+    assert _worst(got[:R], want) < 3e-2  # roundings alone: a row or column of 260 values or more is within a few times the whole
+
+
+@pytest.mark.parametrize("qtype,rows,expected,groups,most,N,K,tn,splits", [
+    ("Q4_K", 800, 0, 8, 400, 28672, 4096, 128, 1),   # 100 rows to a group: a tile of 256 would be emptier
+    ("BF16", 800, 0, 8, 400, 4096, 14336, 128, 1),   # ... and not split along K
+    ("Q4_K", 1200, 0, 8, 600, 28672, 4096, 256, 1),
+    ("Q4_K", 400, 100, 2, 200, 28672, 4096, 128, 1),  # one rank of four: its experts get a quarter of the step's rows
+    ("BF16", 2, 0, 8, 1, 28672, 4096, 16, 1),        # one token, short rows: not split
+    ("Q4_K", 1024, 0, 128, 128, 2048, 768, 32, 1)])  # many experts in four bits: 32 tokens at least
+def test_grouped_rows_plans(C, qtype, rows, expected, groups, most, N, K, tn, splits):
+    import ctypes
+
+    out = (ctypes.c_int * 4)()
+    assert C.lib().oxb_gemm_grouped_rows_plan(rows, C.QTYPE_CODE[qtype], groups, most, expected, N, K, out) == 0
+    assert (out[0], out[3]) == (tn, splits)
