@@ -397,10 +397,12 @@ struct GroupArgs {
   // fetched from HBM once.  The grid has room for the longest list that the rows can make (gathered_tiles); CTAs past
   // its end leave at once.  (A grid of every group's possible tiles would be mostly CTAs that leave: 3 of 4 at a
   // prefill of 8 experts, 4 of 5 at 128 experts with a tile fitted to their few rows.)
+  // by_group: one group's weight tiles after another's instead (blockIdx.x = place in the list times weight tiles, in a group
+  // the token tiles innermost), see gathered_plan.
   // Other grouped launches: blockIdx.z = g * t_tiles + token tile.
   const int* row_offsets;
   int t_tiles;
-  int n_groups;  // gathered groups only
+  int n_groups, by_group;  // gathered groups only
 };
 
 // Most token tiles that `rows` rows in `groups` groups of at most max_rows rows can make
@@ -474,7 +476,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
   int g_row0 = 0;  // first activation / output row of this group (gathered groups)
   if (gathered) {
     pdl_wait();  // the row lists come from the upstream kernel
-    gathered_tile(gr.row_offsets, gr.n_groups, TN, blockIdx.x, zg, tile_t);
+    const int n_tiles = (N + GEMM_BM - 1) / GEMM_BM;
+    gathered_tile(gr.row_offsets, gr.n_groups, TN, gr.by_group ? blockIdx.x / n_tiles : blockIdx.x, zg, tile_t);
     if (tile_t < 0) {
       pdl_launch_dependents();
       return;
@@ -482,6 +485,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     tile_n = blockIdx.z;
     g_row0 = gr.row_offsets[zg];
     T = gr.row_offsets[zg + 1] - g_row0;  // this group's own row count
+    if (gr.by_group) {
+      const int at = blockIdx.x % n_tiles + tile_t * n_tiles, tiles = (T + TN - 1) / TN;  // place among the group's tiles
+      tile_n = at / tiles;
+      tile_t = at % tiles;
+    }
   }
   if (gr.enabled && !gathered && gr.scale != nullptr) {
     // the routing weights come from the upstream kernel
@@ -1208,6 +1216,11 @@ inline GemmPlan gathered_plan(int rows, int expected, int groups, int max_rows, 
   const GemmPlan p = gemm_plan(most, N, K, 0, sm_count, 1, 0, packed, active);
   return p.splits > 1 && !p.cluster ? gemm_plan(most, N, K, 1, sm_count, 1, 0, packed, active) : p;
 }
+// Order of a gathered launch: group by group where one group's weight tiles fill the SMs and the tiles of tokens are small (8 experts of
+// 28672 x 4096, bf16, 2 to 128 tokens: 84 to 315 us; all groups' tiles for each weight tile, which reads eight streams at once, 96
+// to 330).  With few weight tiles to a group it is the other way round (128 experts of 1536 x 2048, 128 tokens, most to 8
+// of them: 133 and 122), as with tiles of 128 tokens and more (256 tokens: 366 and 354).
+inline bool gathered_by_group(const GemmPlan& p, int groups, int sm_count) { return groups > 1 && p.n_tiles >= sm_count && p.tn <= 64; }
 
 // Largest cluster the kernel instance can be launched with: 16 where the device accepts the
 // non-portable size for this footprint, else the portable 8.
@@ -1244,7 +1257,7 @@ template <int TN, int QT = QT_BF16>
 int gemm_launch(const CUtensorMap& tmW, const CUtensorMap& tmX, __nv_bfloat16* Y, const float* bias, int N, int T, int K,
                 int ldY, const GemmPlan& p, float* ws, int* counters, int epi_mode, const ArArgs& ar,
                 cudaStream_t stream, const QwArgs& qw = QwArgs{nullptr, 0, nullptr, 0},
-                const GroupArgs& gr = GroupArgs{0, 0, 0, 0, nullptr, 0, 0, nullptr, 1, 0}, int groups = 1,
+                const GroupArgs& gr = GroupArgs{0, 0, 0, 0, nullptr, 0, 0, nullptr, 1, 0, 0}, int groups = 1,
                 const RopeArgs& ro = RopeArgs{nullptr, nullptr, nullptr, 0, 0, 0, 0, 0, 0, 0, nullptr, nullptr},
                 const NormArgs& nm = NormArgs{nullptr, 0.f, 0.f, nullptr, nullptr}) {
   using Cfg = GemmTile<TN>;
@@ -1274,7 +1287,8 @@ int gemm_launch(const CUtensorMap& tmW, const CUtensorMap& tmX, __nv_bfloat16* Y
     if (splits > mc) splits = mc;
   }
   dim3 grid(p.n_tiles, splits, gr.enabled ? groups * gr.t_tiles : p.t_tiles);
-  if (gr.row_offsets != nullptr) grid = dim3(p.t_tiles, splits, p.n_tiles);  // p.t_tiles: the list's length
+  if (gr.row_offsets != nullptr)  // p.t_tiles: the list's length
+    grid = gr.by_group ? dim3((unsigned)p.t_tiles * p.n_tiles, splits) : dim3(p.t_tiles, splits, p.n_tiles);
   const dim3 block(QT == QT_BF16 ? GEMM_THREADS : GEMM_THREADS_MMQ);
   cudaError_t le;
   GroupArgs grl = gr;
@@ -1295,7 +1309,7 @@ int gemm_launch(const CUtensorMap& tmW, const CUtensorMap& tmX, __nv_bfloat16* Y
 template <int QT>
 int gemm_launch_mmq(const CUtensorMap& tmX, __nv_bfloat16* Y, const float* bias, int N, int T, int K, int ldY,
                     const GemmPlan& p, float* ws, int* counters, int epi_mode, const ArArgs& ar, cudaStream_t stream,
-                    const QwArgs& qw, const GroupArgs& gr = GroupArgs{0, 0, 0, 0, nullptr, 0, 0, nullptr, 1, 0}, int groups = 1,
+                    const QwArgs& qw, const GroupArgs& gr = GroupArgs{0, 0, 0, 0, nullptr, 0, 0, nullptr, 1, 0, 0}, int groups = 1,
                     const CUtensorMap* tmWq = nullptr) {
   // tmWq: byte map of the packed rows (needed by the staged Q4_K path); other formats never touch tmW
   const CUtensorMap& tmW = tmWq != nullptr ? *tmWq : tmX;

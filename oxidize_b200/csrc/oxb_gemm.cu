@@ -50,7 +50,7 @@ static int gemm_bf16_impl(const void* X, const void* W, void* Y, const float* bi
   ArArgs ar;
   memset(&ar, 0, sizeof(ar));
   const QwArgs qw{nullptr, 0, nullptr, 0, 0};
-  const GroupArgs gr{0, 0, 0, 0, nullptr, 0, 0, nullptr, 1, 0};
+  const GroupArgs gr{0, 0, 0, 0, nullptr, 0, 0, nullptr, 1, 0, 0};
   const RopeArgs ro{nullptr, nullptr, nullptr, 0, 0, 0, 0, 0, 0, 0, nullptr, nullptr};
   switch (p.tn) {
     case 16: return gemm_launch<16>(tmW, tmX, y, bias, N, T, K, ldY, p, wsf, counters, epi_mode, ar, stream, qw, gr, 1, ro, nm);
@@ -143,7 +143,7 @@ OXB_API int oxb_gemm_quant(const void* X, const void* Wq, int qtype, size_t row_
   ArArgs ar;
   memset(&ar, 0, sizeof(ar));
   QwArgs qw{reinterpret_cast<const uint8_t*>(Wq), row_bytes, scales, scale_ld, 0};
-  const GroupArgs g0{0, 0, 0, 0, nullptr, 0, 0, nullptr, 1, 0};
+  const GroupArgs g0{0, 0, 0, 0, nullptr, 0, 0, nullptr, 1, 0, 0};
   return launch_mmq(qtype, Wq, (uint64_t)N, tmX, y, bias, N, T, K, ldY, p, wsf, counters, epi_mode, ar, stream, qw, g0, 1);
 }
 
@@ -190,7 +190,7 @@ static int gemm_ar_impl(const void* X, const void* W, void* Y, const void* resid
   __nv_bfloat16* y = reinterpret_cast<__nv_bfloat16*>(Y);
   float* wsf = reinterpret_cast<float*>(ws);
   const QwArgs qw0{nullptr, 0, nullptr, 0, 0};
-  const GroupArgs gr0{0, 0, 0, 0, nullptr, 0, 0, nullptr, 1, 0};
+  const GroupArgs gr0{0, 0, 0, 0, nullptr, 0, 0, nullptr, 1, 0, 0};
   const RopeArgs ro0{nullptr, nullptr, nullptr, 0, 0, 0, 0, 0, 0, 0, nullptr, nullptr};
   switch (p.tn) {
     case 16: return gemm_launch<16>(tmW, tmX, y, nullptr, N, T, K, ldY, p, wsf, counters, 0, ar, stream, qw0, gr0, 1, ro0, nm);
@@ -242,7 +242,7 @@ static int gemm_qkv_rope_impl(const void* X, const void* W, int T, int K, const 
               reinterpret_cast<__nv_bfloat16*>(kv_data)};
   __nv_bfloat16* y = reinterpret_cast<__nv_bfloat16*>(q_out);  // only its alignment is looked at
   const QwArgs qw{nullptr, 0, nullptr, 0, 0};
-  const GroupArgs gr{0, 0, 0, 0, nullptr, 0, 0, nullptr, 1, 0};
+  const GroupArgs gr{0, 0, 0, 0, nullptr, 0, 0, nullptr, 1, 0, 0};
   switch (p.tn) {
     case 16: return gemm_launch<16>(tmW, tmX, y, nullptr, N, T, K, N, p, nullptr, nullptr, EPI_ROPE, ar, stream, qw, gr, 1, ro, nm);
     case 32: return gemm_launch<32>(tmW, tmX, y, nullptr, N, T, K, N, p, nullptr, nullptr, EPI_ROPE, ar, stream, qw, gr, 1, ro, nm);
@@ -354,7 +354,7 @@ OXB_API int oxb_gemm_grouped(const void* X, int x_rows, const void* W, int qtype
   float* wsf = reinterpret_cast<float*>(ws);
   ArArgs ar;
   memset(&ar, 0, sizeof(ar));
-  GroupArgs gr{1, N, x_rows, y_stride, scale, scale_ld, 0, nullptr, 1, 0};
+  GroupArgs gr{1, N, x_rows, y_stride, scale, scale_ld, 0, nullptr, 1, 0, 0};
   QwArgs qw{reinterpret_cast<const uint8_t*>(W), row_bytes, nullptr, 0, 0};
   if (qtype == QT_BF16) {
     e = oxb_make_tmap_2d(&tmW, W, (uint64_t)groups * N, K, (uint64_t)K * 2, GEMM_BM, GEMM_BK, 2);
@@ -394,7 +394,7 @@ OXB_API int oxb_gemm_batched(const void* X, const void* W, void* Y, long long y_
   __nv_bfloat16* y = reinterpret_cast<__nv_bfloat16*>(Y);
   ArArgs ar;
   memset(&ar, 0, sizeof(ar));
-  const GroupArgs gr{1, N, T, y_stride, nullptr, 0, 0, nullptr, p.t_tiles, 0};
+  const GroupArgs gr{1, N, T, y_stride, nullptr, 0, 0, nullptr, p.t_tiles, 0, 0};
   const QwArgs qw{nullptr, 0, nullptr, 0, 0};
   switch (p.tn) {
     case 16: return gemm_launch<16>(tmW, tmX, y, nullptr, N, T, K, ldY, p, nullptr, nullptr, 0, ar, stream, qw, gr, groups);
@@ -440,7 +440,7 @@ OXB_API int oxb_gemm_grouped_rows(const void* X, int rows_cap, const void* W, in
   __nv_bfloat16* y = reinterpret_cast<__nv_bfloat16*>(Y);
   ArArgs ar;
   memset(&ar, 0, sizeof(ar));
-  GroupArgs gr{1, N, 0, 0, nullptr, 0, 0, row_offsets, p.t_tiles, groups};
+  GroupArgs gr{1, N, 0, 0, nullptr, 0, 0, row_offsets, p.t_tiles, groups, gathered_by_group(p, groups, sm_count())};
   QwArgs qw{reinterpret_cast<const uint8_t*>(W), row_bytes, nullptr, 0, 0};
   if (qtype == QT_BF16) {
     e = oxb_make_tmap_2d(&tmW, W, (uint64_t)groups * N, K, (uint64_t)K * 2, GEMM_BM, GEMM_BK, 2);

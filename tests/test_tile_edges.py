@@ -181,9 +181,9 @@ def _worst(got, want):
 
 
 @pytest.mark.parametrize("qtype", ["BF16", "Q4_K"])
-@pytest.mark.parametrize("N,K,rows", [(260, 2624, [300, 130, 0, 257]), (260, 2304, [150] * 5), (300, 2560, [1] * 200 + [40])])
-def test_grouped_rows_wide_tiles(C, qtype, N, K, rows):
-    """Tiles of 256 rows over rows long enough that every ring wraps; groups by the hundred."""
+@pytest.mark.parametrize("N,K,rows", [(260, 2624, [300, 130, 0, 257]), (260, 2304, [150] * 5), (18961, 256, [0, 70, 5, 33, 1]), (300, 2560, [1] * 200 + [40])])
+def test_grouped_rows_wide_tiles_and_orders(C, qtype, N, K, rows):
+    """Tiles of 256 rows over rows long enough that every ring wraps, more weight tiles than SMs (group by group), groups by the hundred."""
     from oxidize_b200.ops import cuda_moe
 
     if qtype == "Q4_K" and K % 256:
