@@ -57,7 +57,7 @@ prefill_pages_kernel(const uint8_t* __restrict__ cache, const float* __restrict_
   const int b = blockIdx.y, page = blockIdx.x;
   const int qlen = query_start[b + 1] - query_start[b], len = seq_lens[b];
   if (qlen < min_rows || page * ATT_PAGE >= len) return;
-  if (window > 0 && (page + 1) * ATT_PAGE <= ((len - qlen - window + 1) & ~(AP_KEYS - 1))) return;  // below the first tile of keys
+  if (window > 0 && (page + 1) * ATT_PAGE <= len - qlen - window + 1) return;  // no row sees any of it
   const int dst_page = prefill_page_base(query_start, seq_lens, min_rows, b) + page;
   if (dst_page >= cap_pages || page >= max_blocks) return;
   int blk = block_tables[(size_t)b * max_blocks + page];
@@ -181,12 +181,14 @@ paged_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         for (int c = 0; c < CH; ++c)
           tma_load_3d(s_q + (t * CH + c) * AP_QCHUNK, &tmQ, &q_full, c * 64, h0, q0 + m0 + t * tok_per);
     }
-    // lane = (page of the tile, column chunk); pages past the last one repeat it (their keys are masked)
+    // lane = (page of the tile, column chunk); pages before the first one that a row sees, which a window may have given back
+    // and whose table entries mean nothing, and past the last one repeat those (their keys are masked)
     const int pg = lane % AP_PAGES, ch = lane / AP_PAGES;
     const int last_page = (seq_len - 1) / ATT_PAGE, first_page = lo / ATT_PAGE;
+    const int first_seen = a.window > 0 ? max(0, pos0 - a.window + 1) / ATT_PAGE : 0;
     const int base = a.block_tables == nullptr ? prefill_page_base(a.query_start, a.seq_lens, a.min_rows, b) : 0;
     auto block_of = [&](int i) {  // cache block of this lane's page in tile i
-      const int p = min(first_page + i * AP_PAGES + pg, last_page);
+      const int p = min(max(first_page + i * AP_PAGES + pg, first_seen), last_page);
       return a.block_tables == nullptr ? base + p : a.block_tables[(size_t)b * a.max_blocks + p];
     };
     int next = block_of(0);

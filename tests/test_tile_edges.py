@@ -214,3 +214,16 @@ def test_grouped_rows_plans(C, qtype, rows, expected, groups, most, N, K, tn, sp
     out = (ctypes.c_int * 4)()
     assert C.lib().oxb_gemm_grouped_rows_plan(rows, C.QTYPE_CODE[qtype], groups, most, expected, N, K, out) == 0
     assert (out[0], out[3]) == (tn, splits)
+
+
+@pytest.mark.parametrize("kvd", ["bf16", "q8"])
+@pytest.mark.parametrize("lens,window", [([(200, 1000), (33, 500)], 50), ([(256, 600), (1, 300)], 100), ([(300, 700)], 17)])
+def test_long_portions_read_no_page_below_the_window(C, kvd, lens, window):
+    """Table entries of pages that no row sees may be anything, and the pages hold anything: here ids out of range."""
+    cpu, meta, gpu, on_gpu, q = _step(kvd, 128, 8, 2, lens)
+    want = ref.paged_attention(q.float(), cpu, 0, meta, 128 ** -0.5, window)
+    for b, (n, c) in enumerate(lens):
+        on_gpu.block_tables[b, : max(0, c - n - window + 1) // 16] = -1 - b
+    got = C.paged_attention(q.cuda(), gpu, 0, on_gpu, 128 ** -0.5, window)
+    _check_status(C)
+    assert _off(got, want) < (2.5e-3 if kvd == "bf16" else 6e-3)  # (as test_long_portions)
