@@ -315,6 +315,27 @@ static __global__ void qk_rope_kvwrite_kernel(const __nv_bfloat16* __restrict__ 
 // loads and stores are 2 V bytes wide and nothing goes through shared memory.  One value per thread and a CTA per head was
 // bound by its CTAs (24576 of them, 26 us, for 512 tokens x 48 heads of 128 into a q8 cache; four layers of a prefill of 512 take 65 us less
 // with this).  The one above stays for other widths and rotations.
+// N neighbouring floats on an N-float boundary
+template <int N>
+__device__ __forceinline__ void load_floats(const float* p, float* o) {
+  if constexpr (N == 1) {
+    o[0] = p[0];
+  } else if constexpr (N == 2) {
+    const float2 x = *reinterpret_cast<const float2*>(p);
+    o[0] = x.x;
+    o[1] = x.y;
+  } else {
+#pragma unroll
+    for (int j = 0; j < N; j += 4) {
+      const float4 x = *reinterpret_cast<const float4*>(p + j);
+      o[j] = x.x;
+      o[j + 1] = x.y;
+      o[j + 2] = x.z;
+      o[j + 3] = x.w;
+    }
+  }
+}
+
 template <int V>
 static __global__ void __launch_bounds__(256)
 qk_rope_kvwrite_warp_kernel(const __nv_bfloat16* __restrict__ qkv, const int* __restrict__ positions, const int* __restrict__ slots,
@@ -324,13 +345,14 @@ qk_rope_kvwrite_warp_kernel(const __nv_bfloat16* __restrict__ qkv, const int* __
   constexpr int HD = 32 * V;
   pdl_launch_dependents();
   pdl_wait();
-  const int heads = nq + 2 * nkv, lane = threadIdx.x & 31, d0 = lane * V;
-  const long long w = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (w >= (long long)T * heads) return;
-  const int t = (int)(w / heads), h = (int)(w % heads);
+  const unsigned heads = nq + 2 * nkv, w = blockIdx.x * 8 + (threadIdx.x >> 5);  // (32 bits: a 64-bit division is a third of a us)
+  const int lane = threadIdx.x & 31, d0 = lane * V;
+  if (w >= T * heads) return;
+  const int t = (int)(w / heads), h = (int)(w - t * heads);
+  const int slot = slots[t], pos = positions[t];  // read along with the row: for few tokens the chain of loads is the kernel's time
   float v[V];
   {
-    const uint32_t* src = reinterpret_cast<const uint32_t*>(qkv + w * HD + d0);
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(qkv + (size_t)w * HD + d0);
     uint32_t r[V / 2];
     if constexpr (V == 2) {
       r[0] = src[0];
@@ -355,35 +377,44 @@ qk_rope_kvwrite_warp_kernel(const __nv_bfloat16* __restrict__ qkv, const int* __
   const bool is_q = h < nq, is_k = !is_q && h < nq + nkv;
   if (is_q || is_k) {
     const float* nw = is_q ? qn : kn;
+    const int p = pos < 0 ? 0 : (pos >= max_pos ? max_pos - 1 : pos);
+    const float* cs = cos_sin + (size_t)p * rot;
+    const int half = rot >> 1;
+    // (all that is read is on its way before the first value is used)
+    const bool first = d0 < half, turned = d0 < rot;  // split halves: half is a multiple of V; adjacent pairs: rot is
+    const int pair = pairing == 0 ? (first ? d0 : d0 - half) : d0 >> 1;
+    float c[V], sn[V], w_n[V];  // (adjacent pairs: V / 2 angles)
+    if (turned) {
+      if (pairing == 0) {
+        load_floats<V>(cs + pair, c);
+        load_floats<V>(cs + half + pair, sn);
+      } else {
+        load_floats<V / 2>(cs + pair, c);
+        load_floats<V / 2>(cs + half + pair, sn);
+      }
+    }
     if (nw != nullptr) {
+      load_floats<V>(nw + d0, w_n);
       float ss = 0.f;
 #pragma unroll
       for (int j = 0; j < V; ++j) ss += v[j] * v[j];
       const float r = rsqrtf(warp_sum(ss) / (float)HD + eps);
 #pragma unroll
-      for (int j = 0; j < V; ++j) v[j] = v[j] * r * nw[d0 + j];
+      for (int j = 0; j < V; ++j) v[j] = v[j] * r * w_n[j];
     }
-    int p = positions[t];
-    p = p < 0 ? 0 : (p >= max_pos ? max_pos - 1 : p);
-    const float* cs = cos_sin + (size_t)p * rot;
-    const int half = rot >> 1;
-    if (pairing == 0) {  // (half is a multiple of V)
-      const bool first = d0 < half, turned = d0 < rot;
-      const int from = !turned ? lane : first ? lane + half / V : lane - half / V, pair = first ? d0 : d0 - half;
+    if (pairing == 0) {
+      const int from = !turned ? lane : first ? lane + half / V : lane - half / V;
 #pragma unroll
       for (int j = 0; j < V; ++j) {
         const float o = __shfl_sync(0xffffffffu, v[j], from);
-        if (turned) {
-          const float c = cs[pair + j], sn = cs[half + pair + j];
-          v[j] = first ? (v[j] * c - o * sn) : (v[j] * c + o * sn);
-        }
+        if (turned) v[j] = first ? (v[j] * c[j] - o * sn[j]) : (v[j] * c[j] + o * sn[j]);
       }
-    } else if (d0 < rot) {  // (rot is a multiple of V)
+    } else if (turned) {
 #pragma unroll
       for (int j = 0; j < V; j += 2) {
-        const float c = cs[(d0 + j) >> 1], sn = cs[half + ((d0 + j) >> 1)], a = v[j], b = v[j + 1];
-        v[j] = a * c - b * sn;
-        v[j + 1] = b * c + a * sn;
+        const float x = v[j], y = v[j + 1];
+        v[j] = x * c[j / 2] - y * sn[j / 2];
+        v[j + 1] = y * c[j / 2] + x * sn[j / 2];
       }
     }
   }
@@ -400,7 +431,6 @@ qk_rope_kvwrite_warp_kernel(const __nv_bfloat16* __restrict__ qkv, const int* __
     put16(q_out + ((size_t)t * nq + h) * HD + d0, bf16s);
     return;
   }
-  const int slot = slots[t];
   if (slot < 0) return;
   const int kvh = is_k ? h - nq : h - nq - nkv;
   const int blk = slot / kv.page, off = slot % kv.page;

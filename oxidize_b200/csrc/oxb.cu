@@ -351,8 +351,10 @@ OXB_API int oxb_qk_rope_kvwrite(const void* qkv, const int* positions, const int
   KvWriteArgs kv{kv_data, kv_scales, kv_mode, page, nkv, num_blocks};
   // a warp to a head: widths of 64, 128 and 256, rotations whose halves (or, adjacent pairs, whole) are whole lanes
   const int V = hd / 32;
-  const uintptr_t at = reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(q_out) | reinterpret_cast<uintptr_t>(kv_data);
-  if ((V == 2 || V == 4 || V == 8) && rot > 0 && rot <= hd && rot % (pairing == 0 ? 2 * V : V) == 0 && (at & 15) == 0) {
+  const uintptr_t at = reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(q_out) | reinterpret_cast<uintptr_t>(kv_data) |
+                       reinterpret_cast<uintptr_t>(cos_sin) | reinterpret_cast<uintptr_t>(q_norm) | reinterpret_cast<uintptr_t>(k_norm);
+  if ((V == 2 || V == 4 || V == 8) && rot > 0 && rot <= hd && rot % (pairing == 0 ? 2 * V : V) == 0 && (at & 15) == 0 &&
+      (long long)T * (nq + 2 * nkv) < (1LL << 31)) {
     const dim3 grid((unsigned)(((long long)T * (nq + 2 * nkv) + 7) / 8));
     auto go = [&](auto kernel) {
       oxb_launch(kernel, grid, dim3(256), 0, stream, reinterpret_cast<const __nv_bfloat16*>(qkv), positions, slots, cos_sin, max_pos, rot,
