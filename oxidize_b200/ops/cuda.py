@@ -518,10 +518,12 @@ PREFILL_ROWS, PREFILL_SURE = 32, 192
 PREFILL_MAX_PAGES = 1 << 14  # ... their pages, where they have to be converted to bf16 first, up to this many in a step
 
 
-def _long_portions(q, kv, layer, meta) -> bool:
-    """Whether the step has portions for the tcgen05 kernel: their sizes are known on the host and it covers their heads."""
+def _long_portions(q, kv, layer, meta, scale) -> bool:
+    """Whether the step has portions for the tcgen05 kernel: their sizes are known on the host and it covers their heads, on
+    boundaries that tensor copies start on, with scores whose order is that of their products."""
     lens = getattr(meta, "host_lens", None)
-    if not lens or len(lens) != meta.seq_lens.shape[0] or kv.page_size != 16 or q.dtype != torch.bfloat16:
+    if (not lens or len(lens) != meta.seq_lens.shape[0] or kv.page_size != 16 or q.dtype != torch.bfloat16
+            or (q.data_ptr() | kv.data[layer].data_ptr()) % 16 or not 0.0 < scale < float("inf") or any(c < n for n, c in lens)):
         return False
     long = [(n, c) for n, c in lens if n >= PREFILL_ROWS]
     nq, hd, nkv = q.shape[1], q.shape[2], kv.spec.heads(layer)
@@ -563,7 +565,7 @@ def paged_attention(q, kv, layer, meta, scale, sliding_window=0, splits: Optiona
     if out is None:
         out = torch.empty_like(q)
     query_len, short_below = max(1, meta.max_query_len), 0
-    if splits is None and softcap == 0.0 and _long_portions(q, kv, layer, meta):
+    if splits is None and softcap == 0.0 and _long_portions(q, kv, layer, meta, scale):
         short_below = PREFILL_ROWS
         _paged_prefill(q, kv, layer, meta, scale, sliding_window, sink, out, out_scale, gate, gate_per_value)
         short = [n for n, _ in meta.host_lens if n < PREFILL_ROWS]

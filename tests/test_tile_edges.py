@@ -227,3 +227,17 @@ def test_long_portions_read_no_page_below_the_window(C, kvd, lens, window):
     got = C.paged_attention(q.cuda(), gpu, 0, on_gpu, 128 ** -0.5, window)
     _check_status(C)
     assert _off(got, want) < (2.5e-3 if kvd == "bf16" else 6e-3)  # (as test_long_portions)
+
+
+@pytest.mark.parametrize("kvd", ["bf16", "q8"])
+@pytest.mark.parametrize("offset,scale", [(2, 0.09), (6, 0.09), (0, 0.0), (0, -0.09), (8, 0.09)])
+def test_long_portions_of_queries_on_any_boundary_and_with_any_scale(C, kvd, offset, scale):
+    """The tcgen05 kernel copies queries from 16-byte boundaries and takes the maximum before it scales: others are served all the same."""
+    cpu, meta, gpu, on_gpu, q = _step(kvd, 128, 8, 2, LONG)
+    room = torch.zeros(q.numel() + 8, dtype=torch.bfloat16, device="cuda")
+    at = room[offset : offset + q.numel()].view(q.shape)
+    at.copy_(q)
+    got = C.paged_attention(at, gpu, 0, on_gpu, scale, 0)
+    _check_status(C)
+    want = ref.paged_attention(q.float(), cpu, 0, meta, scale, 0)
+    assert _off(got, want) < (2.5e-3 if kvd == "bf16" else 6e-3)  # (as test_long_portions)
