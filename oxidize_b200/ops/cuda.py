@@ -67,7 +67,7 @@ class KernelOptions:
     ar_ll_min_world: int = 2  # rank counts from which the fused all-reduce uses the two-shot exchange
     # Packed-weight calls with more tokens than this decode the matrix to a bf16 staging buffer once and run the bf16
     # GEMM on it (every token tile of the fused kernel decodes the weight tile again); 0 = always the fused kernel,
-    # -1 = by encoding (cuda_quant.DECODE_ABOVE).
+    # -1 = by encoding and size (cuda_quant.decode_once).
     mmq_max_tokens: int = -1
     # Checked mode: the op layer's scratch buffers (split-K partials and tickets, split-KV partials, decode staging) sit
     # between canary bands that ``verify_guards()`` checks (``LLM.step`` does so after every step, the kernel tests
