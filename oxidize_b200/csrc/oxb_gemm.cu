@@ -114,6 +114,17 @@ static int launch_mmq(int qtype, const void* W, uint64_t w_rows, const CUtensorM
 }
 
 
+// The plan of oxb_gemm_quant's tensor-core path: token tile, weight tiles, token tiles, splits
+OXB_API int oxb_gemm_quant_plan(int T, int N, int K, int* out4) {
+  if (T <= 0 || N <= 0 || K <= 0) return (int)cudaErrorInvalidValue;
+  const GemmPlan p = gemm_plan(T, N, K, 0, sm_count(), -1, 0, true);
+  out4[0] = p.tn;
+  out4[1] = p.n_tiles;
+  out4[2] = p.t_tiles;
+  out4[3] = p.splits;
+  return 0;
+}
+
 // Y[T, N] = X[T, K] (bf16) · dequant(Wq)[N, K]^T for packed weights (qtype as in quant_blocks.cuh, or
 // 9 = block-scaled fp8 with `scales` [N, scale_ld]).  The blocks are decoded inside the GEMM by its
 // producer warps; nothing is dequantized to global memory.  K must be a multiple of 64.

@@ -241,3 +241,41 @@ def test_long_portions_of_queries_on_any_boundary_and_with_any_scale(C, kvd, off
     _check_status(C)
     want = ref.paged_attention(q.float(), cpu, 0, meta, scale, 0)
     assert _off(got, want) < (2.5e-3 if kvd == "bf16" else 6e-3)  # (as test_long_portions)
+
+
+@pytest.mark.parametrize("qtype", ["Q4_K", "Q6_K", "Q8_0", "NVFP4", "Q4_0", "FP8B"])
+@pytest.mark.parametrize("T,N,K", [(200, 9601, 2560), (500, 9601, 2560), (256, 9700, 2432), (255, 10000, 2944)])
+def test_packed_gemm_tiles_of_256(C, qtype, T, N, K):
+    """Every ring wraps several times (ten super-blocks and more, or an odd number of k-blocks); rows and columns one by one; nothing
+    but the output is written."""
+    import ctypes
+
+    from oxidize_b200.ops import cuda_quant
+
+    if K % 256 and qtype in ("Q4_K", "Q6_K"):
+        K = 2816
+    plan = (ctypes.c_int * 4)()
+    assert C.lib().oxb_gemm_quant_plan(T, N, K, plan) == 0 and plan[0] == 256 and plan[3] == 1
+    gen = torch.Generator(device="cuda").manual_seed(T + K)
+    some = 1201  # distinct rows, repeated: no whole number of tiles
+    w = qtensor_from_dense((torch.randn(some, K, generator=gen, device="cuda") * 0.05).cpu(), qtype, device="cuda")
+    dense = w.to("cpu").dense_cache().double().cuda()
+    again = -(-N // some)
+    w.data = w.data.repeat(again, 1)[:N].contiguous()
+    w.scales = None if w.scales is None else w.scales.repeat(again, 1)[:N].contiguous()
+    w.shape, w._dense = (N, K), None
+    x = torch.randn(T, K, generator=gen, device="cuda").bfloat16()
+    bias = torch.randn(N, generator=gen, device="cuda")
+    room = torch.full((T + 4, N + 27), 7.0, dtype=torch.bfloat16, device="cuda")
+    out = room[2 : T + 2, 8 : N + 8]
+    C.configure(C.KernelOptions(gemv_max_tokens=0, mmq_max_tokens=0))
+    try:
+        (cuda_quant.linear_fp8 if qtype == "FP8B" else cuda_quant.linear_quant)(x, w, out, bias, room.stride(0))
+    finally:
+        C.configure(C.KernelOptions())
+    _check_status(C)
+    want = (x.double() @ dense.t()).repeat(1, again)[:, :N] + bias.double()
+    assert _off(out, want) < 8e-3  # (as test_packed_gemm_tiles)
+    assert _worst(out, want) < 3e-2  # roundings alone: a row or column of 200 values or more is within a few times the whole
+    out.fill_(7.0)
+    assert (room == 7.0).all()
