@@ -45,8 +45,15 @@ struct AttnArgs {
   float* ws_o;   // [B*nkv*max_mtiles*n_cta_splits, 16, hd]
   float* ws_ml;  // [.., 16, 2]
   int* counters; // [B*nkv*max_mtiles] zero-initialised tickets (CTA splits only)
-  int max_rows;  // > 0: sequences that feed this many rows or more are another kernel's
   unsigned long long* trace;  // optional: phase timestamps (globaltimer ns) of CTA (0,0,0), for latency analysis
+};
+
+// Sequences of a step that are another kernel's (bit b of the words: sequence b); a parameter of its own, so that AttnArgs stays in
+// registers.
+constexpr int ATT_SKIP_WORDS = 64;
+struct AttnSkip {
+  int any;
+  uint32_t bits[ATT_SKIP_WORDS];
 };
 
 #define ATT_STAMP(i)                                                                                          \
@@ -228,7 +235,7 @@ __device__ __forceinline__ void attn_merge_rows(const AttnArgs& a, int G, int b,
 // fourth CTA of the q4 form onto an SM).
 template <int HD, int MODE, int NR>
 __global__ void __launch_bounds__(ATT_WARPS * 32, MODE == 0 ? 1 : 3)
-paged_attention_kernel(const AttnArgs a, int G /*q heads per kv head*/) {
+paged_attention_kernel(const AttnArgs a, int G /*q heads per kv head*/, const __grid_constant__ AttnSkip skip) {
   using Page = AttPage<HD, MODE>;
   constexpr int ROWB = Page::ROWB, STAGE_BYTES = Page::STAGE, STAGES = Page::STAGES, NG = Page::NG;
   constexpr int KS = HD / 16;  // k-steps for QK^T
@@ -245,7 +252,7 @@ paged_attention_kernel(const AttnArgs a, int G /*q heads per kv head*/) {
   const int mtile = blockIdx.x / a.n_cta_splits, csplit = blockIdx.x % a.n_cta_splits;
   const int q0 = a.query_start[b], qlen = a.query_start[b + 1] - q0;
   const int seq_len = a.seq_lens[b];
-  if (a.max_rows > 0 && qlen >= a.max_rows) {
+  if (skip.any && (skip.bits[b >> 5] >> (b & 31) & 1)) {
     pdl_wait();
     return;
   }

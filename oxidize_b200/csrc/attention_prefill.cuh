@@ -30,44 +30,57 @@ constexpr int AP_WARP_TMA = 8, AP_WARP_MMA = 9, AP_THREADS = 320;
 struct AttnPrefillArgs {
   const int* query_start;   // [B + 1]
   const int* seq_lens;      // [B]
-  const int* block_tables;  // [B, max_blocks], or null: pages converted by prefill_pages_kernel
+  const int* block_tables;  // [.., max_blocks], or null: pages converted by prefill_pages_kernel
   const float* sink;        // [nq] or null
   __nv_bfloat16* out;       // [T, nq * HD], rows ld_out apart
-  int B, max_blocks, num_blocks, nkv, G, gp, window, min_rows, ld_out;
+  int max_blocks, num_blocks, nkv, G, gp, window, ld_out;
   float out_scale, scale_log2;
   HeadGate gate;
 };
 
-// Pages of the sequences before b that feed at least min_rows rows (where sequence b's converted pages start); whole warp.
-__device__ __forceinline__ int prefill_page_base(const int* query_start, const int* seq_lens, int min_rows, int b) {
-  int n = 0;
-  for (int i = threadIdx.x & 31; i < b; i += 32)
-    if (query_start[i + 1] - query_start[i] >= min_rows) n += (max(seq_lens[i], 0) + ATT_PAGE - 1) / ATT_PAGE;
-  return __reduce_add_sync(0xffffffffu, n);
+// The sequences of a launch, as the host knows them: a step's others cost it nothing.  (A grid of the longest portion's tiles times
+// all sequences is mostly CTAs without work where a portion runs among decoding sequences: one of 4096 tokens of context and 63 of
+// those, 32 key heads, q8, had 524288 CTAs convert 8192 pages.)
+constexpr int AP_SEQS = 64;
+struct AttnPrefillSeqs {
+  int n;
+  int seq[AP_SEQS];             // index in the step
+  int first_item[AP_SEQS + 1];  // of its row tiles in the launch
+  int first_page[AP_SEQS + 1];  // of its converted pages in the buffer
+};
+
+// Where a value lies in ascending starts[0 .. n] (starts[0] <= v < starts[n])
+__device__ __forceinline__ int prefill_find(const int (&starts)[AP_SEQS + 1], int n, int v) {
+  int i = 0;
+  while (i + 1 < n && starts[i + 1] <= v) ++i;
+  return i;
+}
+// First page that any row of a sequence sees
+__host__ __device__ __forceinline__ int prefill_first_page(int rows, int ctx, int window) {
+  const int key = ctx - rows - window + 1;
+  return window > 0 && key > 0 ? key / ATT_PAGE : 0;
 }
 
-// f16 / q8 / q4 pages of the long sequences as bf16 pages, a CTA for every page and head: out [pages, nkv, K | V, 16, HD].
+// f16 / q8 / q4 pages of the launch's sequences as bf16 pages, a CTA for every page and head: out [pages, nkv, K | V, 16, HD].
 template <int HD, int MODE>
 static __global__ void __launch_bounds__(256)
 prefill_pages_kernel(const uint8_t* __restrict__ cache, const float* __restrict__ scales, const int* __restrict__ query_start,
                      const int* __restrict__ seq_lens, const int* __restrict__ block_tables, int max_blocks, int num_blocks, int nkv,
-                     int window, int min_rows, int cap_pages, __nv_bfloat16* __restrict__ out) {
+                     int window, const __grid_constant__ AttnPrefillSeqs ls, __nv_bfloat16* __restrict__ out) {
   pdl_launch_dependents();
   pdl_wait();
-  const int b = blockIdx.y, page = blockIdx.x;
-  const int qlen = query_start[b + 1] - query_start[b], len = seq_lens[b];
-  if (qlen < min_rows || page * ATT_PAGE >= len) return;
-  if (window > 0 && (page + 1) * ATT_PAGE <= len - qlen - window + 1) return;  // no row sees any of it
-  const int dst_page = prefill_page_base(query_start, seq_lens, min_rows, b) + page;
-  if (dst_page >= cap_pages || page >= max_blocks) return;
+  const int dst_page = ls.first_page[0] + blockIdx.x, at = prefill_find(ls.first_page, ls.n, dst_page), b = ls.seq[at];
+  const int len = seq_lens[b];
+  const int page = prefill_first_page(query_start[b + 1] - query_start[b], len, window) + dst_page - ls.first_page[at];
+  if (page * ATT_PAGE >= len || page >= max_blocks) return;
   int blk = block_tables[(size_t)b * max_blocks + page];
   if ((unsigned)blk >= (unsigned)num_blocks) {
     if (threadIdx.x == 0) oxb_report(OXB_BAD_BLOCK_ID, blk);
     blk = 0;
   }
   const int rows = 2 * ATT_PAGE;  // of this head
-  const size_t row0 = ((size_t)blk * nkv + blockIdx.z) * rows;
-  __nv_bfloat16* o = out + ((size_t)dst_page * nkv + blockIdx.z) * rows * HD;
+  const size_t row0 = ((size_t)blk * nkv + blockIdx.y) * rows;
+  __nv_bfloat16* o = out + ((size_t)dst_page * nkv + blockIdx.y) * rows * HD;
   for (int c = threadIdx.x; c < rows * (HD / 8); c += 256) {  // 8 values
     const int row = c / (HD / 8), col = (c % (HD / 8)) * 8;
     float v[8];
@@ -114,7 +127,8 @@ constexpr int attn_prefill_smem() {
 
 template <int HD>
 __global__ void __launch_bounds__(AP_THREADS, 1)
-paged_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmKV, const AttnPrefillArgs a) {
+paged_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmKV, const AttnPrefillArgs a,
+                     const __grid_constant__ AttnPrefillSeqs ls) {
   constexpr int CH = HD / 64;
   extern __shared__ uint8_t ap_raw[];
   __shared__ uint64_t q_full, k_full[AP_STAGES], k_empty[AP_STAGES], v_full[AP_STAGES], v_empty[AP_STAGES], s_full[2][2],
@@ -122,14 +136,14 @@ paged_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   __shared__ uint32_t tmem_slot;
   __shared__ volatile int abort_flag;
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-  const int b = blockIdx.z, h0 = blockIdx.y * a.gp;  // first query head of this CTA
+  const int at = prefill_find(ls.first_item, ls.n, blockIdx.x), b = ls.seq[at], h0 = blockIdx.y * a.gp;  // first query head of this CTA
   const int kvh = h0 / a.G;
   const int q0 = a.query_start[b], qlen = a.query_start[b + 1] - q0;
   const int tok_per = AP_M / a.gp;  // tokens of a tile
   // (the last rows have the longest way to go: they start first)
-  const int m0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * 2 * tok_per;
+  const int m0 = (ls.first_item[at + 1] - 1 - (int)blockIdx.x) * 2 * tok_per;
   const int seq_len = a.seq_lens[b];
-  if (m0 >= qlen || qlen < a.min_rows || seq_len < qlen) {
+  if (m0 >= qlen || seq_len < qlen) {
     pdl_wait();
     return;
   }
@@ -186,7 +200,7 @@ paged_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     const int pg = lane % AP_PAGES, ch = lane / AP_PAGES;
     const int last_page = (seq_len - 1) / ATT_PAGE, first_page = lo / ATT_PAGE;
     const int first_seen = a.window > 0 ? max(0, pos0 - a.window + 1) / ATT_PAGE : 0;
-    const int base = a.block_tables == nullptr ? prefill_page_base(a.query_start, a.seq_lens, a.min_rows, b) : 0;
+    const int base = ls.first_page[at] - prefill_first_page(qlen, seq_len, a.window);  // (converted pages)
     auto block_of = [&](int i) {  // cache block of this lane's page in tile i
       const int p = min(max(first_page + i * AP_PAGES + pg, first_seen), last_page);
       return a.block_tables == nullptr ? base + p : a.block_tables[(size_t)b * a.max_blocks + p];

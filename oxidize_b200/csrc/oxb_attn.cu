@@ -15,7 +15,7 @@ OXB_API int oxb_attn_ws_floats(int B, int nkv, int max_mtiles, int n_cta_splits,
 }
 
 template <int HD, int MODE, int NR>
-static int attn_launch_rows(const AttnArgs& a, int B, int G, cudaStream_t stream) {
+static int attn_launch_rows(const AttnArgs& a, const AttnSkip& skip, int B, int G, cudaStream_t stream) {
   constexpr int smem = AttPage<HD, MODE>::SMEM;
   static bool configured = false;
   if (!configured) {
@@ -27,27 +27,35 @@ static int attn_launch_rows(const AttnArgs& a, int B, int G, cudaStream_t stream
   // (The KV splits of a row tile stay independent CTAs and the last one to finish merges: inside a thread-block
   // cluster every CTA would wait for the slowest split.)
   if (a.n_cta_splits > 1 && (a.ws_o == nullptr || a.ws_ml == nullptr || a.counters == nullptr)) return (int)cudaErrorInvalidValue;
-  oxb_launch(paged_attention_kernel<HD, MODE, NR>, grid, dim3(ATT_WARPS * 32), (size_t)smem, stream, a, G);
+  oxb_launch(paged_attention_kernel<HD, MODE, NR>, grid, dim3(ATT_WARPS * 32), (size_t)smem, stream, a, G, skip);
   OXB_CHECK_LAUNCH();
   return 0;
 }
 
 template <int HD, int MODE = 0>
-static int attn_launch(const AttnArgs& a, int B, int G, int max_query_len, cudaStream_t stream) {
+static int attn_launch(const AttnArgs& a, const AttnSkip& skip, int B, int G, int max_query_len, cudaStream_t stream) {
   if constexpr (HD == 64 || HD == 128) {
-    if (max_query_len * G <= 8) return attn_launch_rows<HD, MODE, 1>(a, B, G, stream);
+    if (max_query_len * G <= 8) return attn_launch_rows<HD, MODE, 1>(a, skip, B, G, stream);
   }
-  return attn_launch_rows<HD, MODE, 2>(a, B, G, stream);
+  return attn_launch_rows<HD, MODE, 2>(a, skip, B, G, stream);
 }
 
-static int paged_attention(const void* q, void* out, const void* kv_data, const float* kv_scales, const int* block_tables,
-                           const int* seq_lens, const int* query_start, int B, int max_blocks, int nq, int nkv, int hd, int kv_mode,
-                           int max_query_len, int n_cta_splits, int window, float scale, float softcap, const float* sink, int ld_out,
-                           float out_scale, float* ws_o, float* ws_ml, int* counters, int num_blocks, const void* gate, int ld_gate,
-                           int gate_per_value, int max_rows, cudaStream_t stream) {
+// skip (host, skip_words words, or null): bit b of it leaves sequence b alone, whose rows are another kernel's (max_query_len: of the
+// others).
+OXB_API int oxb_paged_attention(const void* q, void* out, const void* kv_data, const float* kv_scales,
+                                const int* block_tables, const int* seq_lens, const int* query_start, int B,
+                                int max_blocks, int nq, int nkv, int hd, int kv_mode, int max_query_len,
+                                int n_cta_splits, int window, float scale, float softcap, const float* sink, int ld_out,
+                                float out_scale, float* ws_o, float* ws_ml, int* counters, int num_blocks,
+                                const void* gate, int ld_gate, int gate_per_value, const uint32_t* skip_bits, int skip_words,
+                                cudaStream_t stream) {
   if (B <= 0) return 0;
   if (nq % nkv != 0 || (gate != nullptr && gate_per_value && (ld_gate % 2 != 0 || (reinterpret_cast<uintptr_t>(gate) & 3) != 0)))
     return (int)cudaErrorInvalidValue;
+  AttnSkip skip;
+  skip.any = skip_bits != nullptr && skip_words > 0;
+  if (skip.any && (skip_words > ATT_SKIP_WORDS || B > 32 * skip_words)) return (int)cudaErrorInvalidValue;
+  for (int i = 0; i < ATT_SKIP_WORDS; ++i) skip.bits[i] = skip.any && i < skip_words ? skip_bits[i] : 0;
   const int G = nq / nkv;
   AttnArgs a;
   a.q = reinterpret_cast<const __nv_bfloat16*>(q);
@@ -75,56 +83,31 @@ static int paged_attention(const void* q, void* out, const void* kv_data, const 
   a.ws_ml = ws_ml;
   a.counters = counters;
   a.num_blocks = num_blocks;
-  a.max_rows = max_rows;
   a.trace = g_oxb_attn_trace;
-  if (kv_mode == 2 && hd == 128) return attn_launch<128, 2>(a, B, G, max_query_len, stream);
-  if (kv_mode == 2 && hd == 64) return attn_launch<64, 2>(a, B, G, max_query_len, stream);
-  if (kv_mode == 3 && hd == 128) return attn_launch<128, 3>(a, B, G, max_query_len, stream);
-  if (kv_mode == 3 && hd == 64) return attn_launch<64, 3>(a, B, G, max_query_len, stream);
-  if (hd == 128) return attn_launch<128>(a, B, G, max_query_len, stream);
-  if (hd == 64) return attn_launch<64>(a, B, G, max_query_len, stream);
+  if (kv_mode == 2 && hd == 128) return attn_launch<128, 2>(a, skip, B, G, max_query_len, stream);
+  if (kv_mode == 2 && hd == 64) return attn_launch<64, 2>(a, skip, B, G, max_query_len, stream);
+  if (kv_mode == 3 && hd == 128) return attn_launch<128, 3>(a, skip, B, G, max_query_len, stream);
+  if (kv_mode == 3 && hd == 64) return attn_launch<64, 3>(a, skip, B, G, max_query_len, stream);
+  if (hd == 128) return attn_launch<128>(a, skip, B, G, max_query_len, stream);
+  if (hd == 64) return attn_launch<64>(a, skip, B, G, max_query_len, stream);
   if (kv_mode != 0) return (int)cudaErrorInvalidValue;
-  if (hd == 32) return attn_launch<32>(a, B, G, max_query_len, stream);
-  if (hd == 96) return attn_launch<96>(a, B, G, max_query_len, stream);
-  if (hd == 192) return attn_launch<192>(a, B, G, max_query_len, stream);
-  if (hd == 256) return attn_launch<256>(a, B, G, max_query_len, stream);
+  if (hd == 32) return attn_launch<32>(a, skip, B, G, max_query_len, stream);
+  if (hd == 96) return attn_launch<96>(a, skip, B, G, max_query_len, stream);
+  if (hd == 192) return attn_launch<192>(a, skip, B, G, max_query_len, stream);
+  if (hd == 256) return attn_launch<256>(a, skip, B, G, max_query_len, stream);
   return (int)cudaErrorInvalidValue;
 }
-
-OXB_API int oxb_paged_attention(const void* q, void* out, const void* kv_data, const float* kv_scales,
-                                const int* block_tables, const int* seq_lens, const int* query_start, int B,
-                                int max_blocks, int nq, int nkv, int hd, int kv_mode, int max_query_len,
-                                int n_cta_splits, int window, float scale, float softcap, const float* sink, int ld_out,
-                                float out_scale, float* ws_o, float* ws_ml, int* counters, int num_blocks,
-                                const void* gate, int ld_gate, int gate_per_value, cudaStream_t stream) {
-  return paged_attention(q, out, kv_data, kv_scales, block_tables, seq_lens, query_start, B, max_blocks, nq, nkv, hd, kv_mode,
-                         max_query_len, n_cta_splits, window, scale, softcap, sink, ld_out, out_scale, ws_o, ws_ml, counters,
-                         num_blocks, gate, ld_gate, gate_per_value, 0, stream);
-}
-
-// The same for the sequences that feed fewer than max_rows rows (max_query_len: the most of those); the others are left alone.
-OXB_API int oxb_paged_attention_short(const void* q, void* out, const void* kv_data, const float* kv_scales,
-                                      const int* block_tables, const int* seq_lens, const int* query_start, int B,
-                                      int max_blocks, int nq, int nkv, int hd, int kv_mode, int max_query_len,
-                                      int n_cta_splits, int window, float scale, float softcap, const float* sink, int ld_out,
-                                      float out_scale, float* ws_o, float* ws_ml, int* counters, int num_blocks,
-                                      const void* gate, int ld_gate, int gate_per_value, int max_rows, cudaStream_t stream) {
-  return paged_attention(q, out, kv_data, kv_scales, block_tables, seq_lens, query_start, B, max_blocks, nq, nkv, hd, kv_mode,
-                         max_query_len, n_cta_splits, window, scale, softcap, sink, ld_out, out_scale, ws_o, ws_ml, counters,
-                         num_blocks, gate, ld_gate, gate_per_value, max_rows, stream);
-}
-
 
 // ----------------------------------------------------------------------------- long portions
 template <int HD>
 static int prefill_convert(int mode, const void* kv_data, const float* kv_scales, const int* block_tables, const int* seq_lens,
-                           const int* query_start, int B, int max_blocks, int num_blocks, int nkv, int max_pages, int cap_pages,
-                           int window, int min_rows, __nv_bfloat16* pages, cudaStream_t stream) {
+                           const int* query_start, int max_blocks, int num_blocks, int nkv, int window, const AttnPrefillSeqs& ls,
+                           __nv_bfloat16* pages, cudaStream_t stream) {
   const uint8_t* src = reinterpret_cast<const uint8_t*>(kv_data);
-  const dim3 grid(max_pages, B, nkv), block(256);
+  const dim3 grid(ls.first_page[ls.n] - ls.first_page[0], nkv), block(256);
   auto go = [&](auto kernel) {
     return oxb_launch(kernel, grid, block, 0, stream, src, kv_scales, query_start, seq_lens, block_tables, max_blocks, num_blocks, nkv,
-                      window, min_rows, cap_pages, pages);
+                      window, ls, pages);
   };
   const cudaError_t e = mode == 1 ? go(prefill_pages_kernel<HD, 1>) : mode == 2 ? go(prefill_pages_kernel<HD, 2>) : go(prefill_pages_kernel<HD, 3>);
   if (e != cudaSuccess) return (int)e;
@@ -133,7 +116,8 @@ static int prefill_convert(int mode, const void* kv_data, const float* kv_scales
 }
 
 template <int HD>
-static int prefill_launch(const void* q, const void* pages, AttnPrefillArgs a, int T, int nq, int max_query_len, cudaStream_t stream) {
+static int prefill_launch(const void* q, const void* pages, const AttnPrefillArgs& a, const AttnPrefillSeqs& ls, int T, int nq,
+                          cudaStream_t stream) {
   static bool configured[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -151,9 +135,8 @@ static int prefill_launch(const void* q, const void* pages, AttnPrefillArgs a, i
   if (e) return e;
   e = oxb_make_tmap_2d(&tkv, pages, (uint64_t)a.num_blocks * a.nkv * 2 * ATT_PAGE, HD, (uint64_t)HD * 2, ATT_PAGE, 64, 2);
   if (e) return e;
-  const int tok_per_cta = 2 * AP_M / a.gp;
-  const dim3 grid((max_query_len + tok_per_cta - 1) / tok_per_cta, nq / a.gp, a.B);
-  const cudaError_t le = oxb_launch(paged_prefill_kernel<HD>, grid, dim3(AP_THREADS), (size_t)attn_prefill_smem<HD>(), stream, tq, tkv, a);
+  const dim3 grid(ls.first_item[ls.n], nq / a.gp);
+  const cudaError_t le = oxb_launch(paged_prefill_kernel<HD>, grid, dim3(AP_THREADS), (size_t)attn_prefill_smem<HD>(), stream, tq, tkv, a, ls);
   if (le != cudaSuccess) return (int)le;
   OXB_CHECK_LAUNCH();
   return 0;
@@ -164,33 +147,25 @@ OXB_API int oxb_paged_prefill_supported(int hd, int nq, int nkv) {
   return (hd == 64 || hd == 128) && nkv > 0 && nq % nkv == 0 && nq <= 65535;
 }
 
-// Attention of the sequences that feed at least min_rows rows (the others are left alone), arguments as oxb_paged_attention.
-// kv_mode > 0: `pages` [cap_pages, nkv, 2, 16, hd] bf16 receives their pages decoded (max_pages: of the longest context).
+// Attention of some sequences of a step (the others are left alone), arguments as oxb_paged_attention: `count` of them, with their
+// index, rows and context length (host arrays; the last two bound the launches, the kernels go by the device's).  scale > 0.
+// kv_mode > 0: `pages` [cap_pages, nkv, 2, 16, hd] bf16 receives the pages that their rows see, decoded.
 OXB_API int oxb_paged_prefill(const void* q, void* out, const void* kv_data, const float* kv_scales, const int* block_tables,
-                              const int* seq_lens, const int* query_start, int B, int T, int max_blocks, int nq, int nkv, int hd,
-                              int kv_mode, int max_query_len, int min_rows, int window, float scale, const float* sink, int ld_out,
-                              float out_scale, int num_blocks, const void* gate, int ld_gate, int gate_per_value, void* pages,
-                              int cap_pages, int max_pages, cudaStream_t stream) {
-  if (B <= 0 || T <= 0 || max_query_len <= 0) return 0;
-  if (!oxb_paged_prefill_supported(hd, nq, nkv) || B > 65535 || kv_mode < 0 || kv_mode > 3 || ld_out % 2 != 0 ||
-      (kv_mode > 0 && (pages == nullptr || cap_pages <= 0 || max_pages <= 0)) ||
+                              const int* seq_lens, const int* query_start, int T, int max_blocks, int nq, int nkv, int hd,
+                              int kv_mode, const int* seqs, const int* rows, const int* ctx, int count, int window, float scale,
+                              const float* sink, int ld_out, float out_scale, int num_blocks, const void* gate, int ld_gate,
+                              int gate_per_value, void* pages, int cap_pages, cudaStream_t stream) {
+  if (count <= 0 || T <= 0) return 0;
+  if (!oxb_paged_prefill_supported(hd, nq, nkv) || kv_mode < 0 || kv_mode > 3 || ld_out % 2 != 0 || !(scale > 0.f) ||
+      (kv_mode > 0 && pages == nullptr) ||
       (gate != nullptr && gate_per_value && (ld_gate % 2 != 0 || (reinterpret_cast<uintptr_t>(gate) & 3) != 0)))
     return (int)cudaErrorInvalidValue;
-  __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(pages);
-  if (kv_mode > 0) {
-    const int e = hd == 128 ? prefill_convert<128>(kv_mode, kv_data, kv_scales, block_tables, seq_lens, query_start, B, max_blocks, num_blocks,
-                                                   nkv, max_pages, cap_pages, window, min_rows, dst, stream)
-                            : prefill_convert<64>(kv_mode, kv_data, kv_scales, block_tables, seq_lens, query_start, B, max_blocks, num_blocks,
-                                                  nkv, max_pages, cap_pages, window, min_rows, dst, stream);
-    if (e) return e;
-  }
   AttnPrefillArgs a;
   a.query_start = query_start;
   a.seq_lens = seq_lens;
   a.block_tables = kv_mode > 0 ? nullptr : block_tables;
   a.sink = sink;
   a.out = reinterpret_cast<__nv_bfloat16*>(out);
-  a.B = B;
   a.max_blocks = max_blocks;
   a.num_blocks = kv_mode > 0 ? cap_pages : num_blocks;
   a.nkv = nkv;
@@ -198,12 +173,40 @@ OXB_API int oxb_paged_prefill(const void* q, void* out, const void* kv_data, con
   a.gp = 1;
   while (a.gp < AP_M && a.G % (2 * a.gp) == 0) a.gp *= 2;  // the largest power of two that divides the group
   a.window = window;
-  a.min_rows = min_rows;
   a.ld_out = ld_out;
   a.out_scale = out_scale;
   a.scale_log2 = scale * 1.4426950408889634f;
   a.gate = HeadGate{gate, ld_gate, gate_per_value};
+  const int tok_per_cta = 2 * AP_M / a.gp;
+  __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(pages);
   const void* src = kv_mode > 0 ? pages : kv_data;
-  return hd == 128 ? prefill_launch<128>(q, src, a, T, nq, max_query_len, stream)
-                   : prefill_launch<64>(q, src, a, T, nq, max_query_len, stream);
+  int page = 0;  // of the buffer
+  for (int at = 0; at < count; at += AP_SEQS) {
+    AttnPrefillSeqs ls;
+    ls.n = count - at < AP_SEQS ? count - at : AP_SEQS;
+    int item = 0;
+    for (int i = 0; i <= AP_SEQS; ++i) {  // (entries past the last sequence repeat the ends)
+      ls.first_item[i] = item;
+      ls.first_page[i] = page;
+      if (i == AP_SEQS) break;
+      ls.seq[i] = 0;
+      if (i >= ls.n) continue;
+      const int n = rows[at + i], c = ctx[at + i];
+      if (n <= 0 || c < n) return (int)cudaErrorInvalidValue;
+      ls.seq[i] = seqs[at + i];
+      item += (n + tok_per_cta - 1) / tok_per_cta;
+      if (kv_mode > 0) page += (c + ATT_PAGE - 1) / ATT_PAGE - prefill_first_page(n, c, window);
+    }
+    if (kv_mode > 0) {
+      if (page > cap_pages) return (int)cudaErrorInvalidValue;
+      const int e = hd == 128 ? prefill_convert<128>(kv_mode, kv_data, kv_scales, block_tables, seq_lens, query_start, max_blocks, num_blocks,
+                                                     nkv, window, ls, dst, stream)
+                              : prefill_convert<64>(kv_mode, kv_data, kv_scales, block_tables, seq_lens, query_start, max_blocks, num_blocks,
+                                                    nkv, window, ls, dst, stream);
+      if (e) return e;
+    }
+    const int e = hd == 128 ? prefill_launch<128>(q, src, a, ls, T, nq, stream) : prefill_launch<64>(q, src, a, ls, T, nq, stream);
+    if (e) return e;
+  }
+  return 0;
 }

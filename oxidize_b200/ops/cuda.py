@@ -122,9 +122,9 @@ def _declare(L) -> None:
     L.oxb_qk_rope_kvwrite.argtypes = [vp, vp, vp, vp, i32, i32, i32, vp, vp, f32, i32, i32, i32, i32, vp, vp, vp, i32,
                                       i32, i32, vp]
     L.oxb_argmax.argtypes = [vp, i32, i32, i32, i32, vp, vp, i32, vp]
-    L.oxb_paged_attention_short.argtypes = [vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, f32, f32,
-                                      vp, i32, f32, vp, vp, vp, i32, vp, i32, i32, i32, vp]
-    L.oxb_paged_prefill.argtypes = [vp] * 7 + [i32] * 10 + [f32, vp, i32, f32, i32, vp, i32, i32, vp, i32, i32, vp]
+    L.oxb_paged_attention.argtypes = [vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, f32, f32,
+                                      vp, i32, f32, vp, vp, vp, i32, vp, i32, i32, vp, i32, vp]
+    L.oxb_paged_prefill.argtypes = [vp] * 7 + [i32] * 6 + [vp] * 3 + [i32] * 2 + [f32, vp, i32, f32, i32, vp, i32, i32, vp, i32, vp]
     L.oxb_paged_prefill_supported.argtypes = [i32] * 3
     L.oxb_sample.argtypes = [vp, i32, i32, i32, vp, vp, vp, vp, vp, i32, vp, vp]
     L.oxb_gemm_quant.argtypes =[vp, vp, i32, sz, vp, i32, vp, vp, i32, i32, i32, i32, i32, i32, vp, sz, vp, i32, vp]
@@ -516,41 +516,45 @@ def attn_splits(B: int, nkv: int, mtiles: int, max_seq_len: int, sms: int, per_s
 # 169 against 85 us; four of them 214 against 411): there the estimates decide, 1.3 us per 64 keys and wave of CTAs, and 100 TFLOP/s.
 PREFILL_ROWS, PREFILL_SURE = 32, 192
 PREFILL_MAX_PAGES = 1 << 14  # ... their pages, where they have to be converted to bf16 first, up to this many in a step
+ATTN_SKIP_WORDS = 64  # sequences of a step that the mma.sync kernel can be told apart, by 32
 
 
-def _long_portions(q, kv, layer, meta, scale) -> bool:
-    """Whether the step has portions for the tcgen05 kernel: their sizes are known on the host and it covers their heads, on
+def _long_portions(q, kv, layer, meta, scale) -> List[int]:
+    """Sequences of the step for the tcgen05 kernel: their sizes are known on the host and it covers their heads, on
     boundaries that tensor copies start on, with scores whose order is that of their products."""
     lens = getattr(meta, "host_lens", None)
-    if (not lens or len(lens) != meta.seq_lens.shape[0] or kv.page_size != 16 or q.dtype != torch.bfloat16
-            or (q.data_ptr() | kv.data[layer].data_ptr()) % 16 or not 0.0 < scale < float("inf") or any(c < n for n, c in lens)):
-        return False
-    long = [(n, c) for n, c in lens if n >= PREFILL_ROWS]
+    if (not lens or len(lens) != meta.seq_lens.shape[0] or len(lens) > 32 * ATTN_SKIP_WORDS or kv.page_size != 16
+            or q.dtype != torch.bfloat16 or (q.data_ptr() | kv.data[layer].data_ptr()) % 16 or not 0.0 < scale < float("inf")):
+        return []
+    take = [i for i, (n, c) in enumerate(lens) if n >= PREFILL_ROWS and c >= n]
+    long = [lens[i] for i in take]
     nq, hd, nkv = q.shape[1], q.shape[2], kv.spec.heads(layer)
     if not long or (kv.dtype_name != "bf16" and sum((c + 15) // 16 for _, c in long) > PREFILL_MAX_PAGES):
-        return False
+        return []
     if max(n for n, _ in long) < PREFILL_SURE:
         ctas = sum(-(-n * nq // 256) for n, _ in long)
         here = 1.3 * -(-ctas // sm_count(q.device)) * (max(c for _, c in long) / 64 + 6) + 6
         if here > sum(4e-8 * nq * hd * n * (c - n / 2) for n, c in long) + 8:
-            return False
-    return bool(lib().oxb_paged_prefill_supported(hd, nq, nkv))
+            return []
+    return take if lib().oxb_paged_prefill_supported(hd, nq, nkv) else []
 
 
-def _paged_prefill(q, kv, layer, meta, scale, window, sink, out, out_scale, gate, gate_per_value) -> None:
+def _paged_prefill(q, kv, layer, meta, take, scale, window, sink, out, out_scale, gate, gate_per_value) -> None:
     T, nq, hd = q.shape
     nkv = kv.spec.heads(layer)
-    long = [(n, c) for n, c in meta.host_lens if n >= PREFILL_ROWS]
+    take = sorted(take, key=lambda i: -meta.host_lens[i][1])  # the longest ways first
+    rows, ctx = ([meta.host_lens[i][j] for i in take] for j in (0, 1))
     pages, cap = None, 0
     if kv.dtype_name != "bf16":
-        cap = sum((c + 15) // 16 for _, c in long)
+        cap = sum((c + 15) // 16 for c in ctx)
         pages = torch.empty(cap, nkv, 2, 16, hd, dtype=torch.bfloat16, device=q.device)
+    ints = ctypes.c_int * len(take)
     _check(lib().oxb_paged_prefill(q.data_ptr(), out.data_ptr(), kv.data[layer].data_ptr(), _p(kv.scales[layer]),
-                                   meta.block_tables.data_ptr(), meta.seq_lens.data_ptr(), meta.query_start.data_ptr(),
-                                   meta.seq_lens.shape[0], T, meta.block_tables.stride(0), nq, nkv, hd, KV_MODE[kv.dtype_name],
-                                   max(n for n, _ in long), PREFILL_ROWS, window, scale, _p(sink), out.stride(0), out_scale,
-                                   kv.num_blocks, _p(gate), 0 if gate is None else gate.stride(0), int(gate_per_value), _p(pages), cap,
-                                   max((c + 15) // 16 for _, c in long), _stream()), "oxb_paged_prefill")
+                                   meta.block_tables.data_ptr(), meta.seq_lens.data_ptr(), meta.query_start.data_ptr(), T,
+                                   meta.block_tables.stride(0), nq, nkv, hd, KV_MODE[kv.dtype_name], ints(*take), ints(*rows), ints(*ctx),
+                                   len(take), window, scale, _p(sink), out.stride(0), out_scale, kv.num_blocks, _p(gate),
+                                   0 if gate is None else gate.stride(0), int(gate_per_value), _p(pages), cap, _stream()),
+           "oxb_paged_prefill")
 
 
 def paged_attention(q, kv, layer, meta, scale, sliding_window=0, splits: Optional[int] = None, softcap: float = 0.0,
@@ -564,20 +568,24 @@ def paged_attention(q, kv, layer, meta, scale, sliding_window=0, splits: Optiona
     G = nq // nkv
     if out is None:
         out = torch.empty_like(q)
-    query_len, short_below = max(1, meta.max_query_len), 0
-    if splits is None and softcap == 0.0 and _long_portions(q, kv, layer, meta, scale):
-        short_below = PREFILL_ROWS
-        _paged_prefill(q, kv, layer, meta, scale, sliding_window, sink, out, out_scale, gate, gate_per_value)
-        short = [n for n, _ in meta.host_lens if n < PREFILL_ROWS]
-        if not short:
+    query_len, seqs, skip = max(1, meta.max_query_len), B, None
+    take = _long_portions(q, kv, layer, meta, scale) if splits is None and softcap == 0.0 else []
+    if take:
+        _paged_prefill(q, kv, layer, meta, take, scale, sliding_window, sink, out, out_scale, gate, gate_per_value)
+        if len(take) == B:
             return out
-        query_len = max(1, max(short))
+        bits = 0
+        for i in take:
+            bits |= 1 << i
+        skip = (ctypes.c_uint32 * ((B + 31) // 32)).from_buffer_copy(bits.to_bytes((B + 31) // 32 * 4, "little"))
+        taken = set(take)
+        query_len, seqs = max(1, max(n for i, (n, _) in enumerate(meta.host_lens) if i not in taken)), B - len(take)
     mtiles = (query_len * G + 15) // 16
     if splits is None:
         span = meta.max_seq_len or kv.page_size
         if sliding_window > 0:
             span = min(span, sliding_window + query_len)
-        splits = attn_splits(B, nkv, mtiles, span, sm_count(q.device), 3 if kv.dtype_name in ("q8", "q4") else 2)
+        splits = attn_splits(seqs, nkv, mtiles, span, sm_count(q.device), 3 if kv.dtype_name in ("q8", "q4") else 2)
     ws_o = ws_ml = cnt = None
     if splits > 1 and B * nkv * mtiles > scratch(q.device).attn_counters.numel():
         splits = 1
@@ -585,13 +593,13 @@ def paged_attention(q, kv, layer, meta, scale, sliding_window=0, splits: Optiona
         tasks = B * nkv * mtiles * splits
         ws_o, ws_ml = scratch(q.device).attn(tasks * 16 * hd, tasks * 32)
         cnt = scratch(q.device).attn_counters
-    _check(lib().oxb_paged_attention_short(q.data_ptr(), out.data_ptr(), kv.data[layer].data_ptr(), _p(kv.scales[layer]),
+    _check(lib().oxb_paged_attention(q.data_ptr(), out.data_ptr(), kv.data[layer].data_ptr(), _p(kv.scales[layer]),
                                      meta.block_tables.data_ptr(), meta.seq_lens.data_ptr(), meta.query_start.data_ptr(),
                                      B, meta.block_tables.stride(0), nq, nkv, hd, KV_MODE[kv.dtype_name],
                                      query_len, splits, sliding_window, scale, float(softcap), _p(sink),
                                      out.stride(0), out_scale, _p(ws_o), _p(ws_ml), _p(cnt), kv.num_blocks, _p(gate),
-                                     0 if gate is None else gate.stride(0), int(gate_per_value), short_below, _stream()),
-           "oxb_paged_attention_short")
+                                     0 if gate is None else gate.stride(0), int(gate_per_value), skip,
+                                     0 if skip is None else len(skip), _stream()), "oxb_paged_attention")
     return out
 
 

@@ -279,3 +279,49 @@ def test_packed_gemm_tiles_of_256(C, qtype, T, N, K):
     assert _worst(out, want) < 3e-2  # roundings alone: a row or column of 200 values or more is within a few times the whole
     out.fill_(7.0)
     assert (room == 7.0).all()
+
+
+def _take(monkeypatch, C, which):
+    """Which sequences the tcgen05 kernel takes, whatever the estimates say."""
+    monkeypatch.setattr(C, "_long_portions", lambda q, kv, layer, meta, *a: [i for i, (n, _) in enumerate(meta.host_lens) if which(i, n)])
+
+
+@pytest.mark.parametrize("kvd,hd,nq,nkv,lens,window", [
+    ("bf16", 128, 8, 2, LONG, 0), ("bf16", 64, 4, 4, LONG, 0), ("bf16", 128, 7, 1, LONG, 50), ("q8", 64, 4, 1, LONG, 90), ("q4", 128, 8, 2, LONG, 0),
+    ("f16", 128, 8, 2, [(40, 400), (1, 30), (64, 64), (33, 1200)], 0), ("q8", 128, 8, 8, [(40, 400), (1, 30), (64, 64), (33, 1200)], 300),
+    ("bf16", 64, 4, 2, [(33 + i % 5, 40 + 3 * i) if i % 9 else (1 + i % 3, 20 + i) for i in range(90)], 0),
+    ("q8", 64, 4, 2, [(33 + i % 5, 40 + 3 * i) if i % 9 else (1 + i % 3, 20 + i) for i in range(90)], 70)])
+@pytest.mark.parametrize("some", [False, True])
+def test_steps_between_the_two_kernels(C, monkeypatch, kvd, hd, nq, nkv, lens, window, some):
+    """All long portions, or every other one, among short ones; more of them than a launch lists, more sequences than a mask word holds."""
+    _take(monkeypatch, C, lambda i, n: n >= 32 and not (some and i % 2))
+    cpu, meta, gpu, on_gpu, q = _step(kvd, hd, nq, nkv, lens)
+    got = C.paged_attention(q.cuda(), gpu, 0, on_gpu, hd ** -0.5, window)
+    _check_status(C)
+    want = ref.paged_attention(q.float(), cpu, 0, meta, hd ** -0.5, window)
+    assert _off(got, want) < (2.5e-3 if kvd == "bf16" else 6e-3)  # (as test_long_portions)
+    off, at = (got.double().cpu() - want.double()).flatten(1), 0
+    for n, _ in lens:  # no sequence is left out
+        assert off[at : at + n].norm() / want[at : at + n].double().norm() < 8e-3
+        at += n
+
+
+@pytest.mark.parametrize("kvd", ["bf16", "q8"])
+@pytest.mark.parametrize("gates", [None, "head", "value"])
+@pytest.mark.parametrize("sinks", [False, True])
+def test_long_portions_with_sinks_and_gates(C, monkeypatch, kvd, gates, sinks):
+    """Against the plain statement: a logit per head in the denominator, a gate per head or per value, a factor on all."""
+    from types import SimpleNamespace
+
+    _take(monkeypatch, C, lambda i, n: n >= 32)
+    cpu, meta, gpu, on_gpu, q = _step(kvd, 128, 8, 2, LONG)
+    gen = torch.Generator().manual_seed(5)
+    sink = torch.randn(8, generator=gen) * 2 if sinks else None
+    gate = None if gates is None else torch.randn(q.shape[0], 8 if gates == "head" else 1024, generator=gen).bfloat16()
+    got = C.paged_attention(q.cuda(), gpu, 0, on_gpu, 128 ** -0.5, sink=None if sink is None else sink.cuda(), out_scale=0.5,
+                            gate=None if gate is None else gate.cuda(), gate_per_value=gates == "value")
+    _check_status(C)
+    want = ref.paged_attention(q.float(), cpu, 0, meta, 128 ** -0.5, sink=sink) * 0.5
+    if gates is not None:
+        want = ref.head_gate(want, gate, SimpleNamespace(heads=8, width=128, gate=gates))
+    assert _off(got, want) < (2.5e-3 if kvd == "bf16" else 6e-3)  # (as test_long_portions)
