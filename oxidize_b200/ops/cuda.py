@@ -13,6 +13,8 @@ from typing import Dict, List, Optional, Sequence, Tuple
 
 import torch
 
+from . import attn_plan
+
 _HERE = os.path.dirname(os.path.abspath(__file__))
 _CSRC = os.path.join(os.path.dirname(_HERE), "csrc")
 LIB_PATH = os.path.join(_CSRC, "liboxb.so")
@@ -499,44 +501,21 @@ def sm_count(device) -> int:
     return _SM_COUNT[idx]
 
 
-def attn_splits(B: int, nkv: int, mtiles: int, max_seq_len: int, sms: int, per_sm: int = 2) -> int:
-    """CTA-level KV splits: as many as keep the grid within ONE wave of ``per_sm`` CTAs per SM (two, or three over
-    quantized pages; a partly filled second wave doubles the kernel's time) while each warp of each split still sees a few
-    pages."""
-    base = max(1, B * nkv * mtiles)
-    want = max(1, (per_sm * sms) // base)
-    pages = max(1, (max_seq_len + 15) // 16)
-    cap = max(1, pages // 8)  # >= 2 pages per warp per split
-    return max(1, min(want, cap, 16))
-
-
-# Long portions take the tcgen05 kernel, which runs 256 (token, head) rows of a key head to a CTA, the other 16 and those split along
-# the keys.  From PREFILL_SURE rows on it is ahead over any context (256 rows over 1000 / 8000, 32 heads / 8: 38 / 176 us against
-# 61 / 281; over none 17 against 27).  Fewer rows leave SMs idle that the other's splits would use (one sequence of 64 over 8000:
-# 169 against 85 us; four of them 214 against 411): there the estimates decide, 1.3 us per 64 keys and wave of CTAs, and 100 TFLOP/s.
-PREFILL_ROWS, PREFILL_SURE = 32, 192
-PREFILL_MAX_PAGES = 1 << 14  # ... their pages, where they have to be converted to bf16 first, up to this many in a step
-ATTN_SKIP_WORDS = 64  # sequences of a step that the mma.sync kernel can be told apart, by 32
-
-
-def _long_portions(q, kv, layer, meta, scale) -> List[int]:
+def _long_portions(q, kv, layer, meta, scale, window) -> List[int]:
     """Sequences of the step for the tcgen05 kernel: their sizes are known on the host and it covers their heads, on
     boundaries that tensor copies start on, with scores whose order is that of their products."""
     lens = getattr(meta, "host_lens", None)
-    if (not lens or len(lens) != meta.seq_lens.shape[0] or len(lens) > 32 * ATTN_SKIP_WORDS or kv.page_size != 16
-            or q.dtype != torch.bfloat16 or (q.data_ptr() | kv.data[layer].data_ptr()) % 16 or not 0.0 < scale < float("inf")):
+    if (not lens or len(lens) != meta.seq_lens.shape[0] or kv.page_size != 16 or q.dtype != torch.bfloat16
+            or (q.data_ptr() | kv.data[layer].data_ptr()) % 16 or not 0.0 < scale < float("inf")):
         return []
-    take = [i for i, (n, c) in enumerate(lens) if n >= PREFILL_ROWS and c >= n]
-    long = [lens[i] for i in take]
     nq, hd, nkv = q.shape[1], q.shape[2], kv.spec.heads(layer)
-    if not long or (kv.dtype_name != "bf16" and sum((c + 15) // 16 for _, c in long) > PREFILL_MAX_PAGES):
+    if not lib().oxb_paged_prefill_supported(hd, nq, nkv):
         return []
-    if max(n for n, _ in long) < PREFILL_SURE:
-        ctas = sum(-(-n * nq // 256) for n, _ in long)
-        here = 1.3 * -(-ctas // sm_count(q.device)) * (max(c for _, c in long) / 64 + 6) + 6
-        if here > sum(4e-8 * nq * hd * n * (c - n / 2) for n, c in long) + 8:
-            return []
-    return take if lib().oxb_paged_prefill_supported(hd, nq, nkv) else []
+    key = ("attention_portions", nq, nkv, hd, kv.dtype_name, window)
+    known = meta.extra.get(key)  # (of an earlier layer of this step)
+    if known is None or known[0] != lens:
+        known = meta.extra[key] = (list(lens), attn_plan.choose(lens, nq, nkv, hd, kv.dtype_name, window, sm_count(q.device)))
+    return known[1]
 
 
 def _paged_prefill(q, kv, layer, meta, take, scale, window, sink, out, out_scale, gate, gate_per_value) -> None:
@@ -568,8 +547,8 @@ def paged_attention(q, kv, layer, meta, scale, sliding_window=0, splits: Optiona
     G = nq // nkv
     if out is None:
         out = torch.empty_like(q)
-    query_len, seqs, skip = max(1, meta.max_query_len), B, None
-    take = _long_portions(q, kv, layer, meta, scale) if splits is None and softcap == 0.0 else []
+    query_len, seqs, skip, span = max(1, meta.max_query_len), B, None, meta.max_seq_len or kv.page_size
+    take = _long_portions(q, kv, layer, meta, scale, sliding_window) if splits is None and softcap == 0.0 else []
     if take:
         _paged_prefill(q, kv, layer, meta, take, scale, sliding_window, sink, out, out_scale, gate, gate_per_value)
         if len(take) == B:
@@ -579,13 +558,13 @@ def paged_attention(q, kv, layer, meta, scale, sliding_window=0, splits: Optiona
             bits |= 1 << i
         skip = (ctypes.c_uint32 * ((B + 31) // 32)).from_buffer_copy(bits.to_bytes((B + 31) // 32 * 4, "little"))
         taken = set(take)
-        query_len, seqs = max(1, max(n for i, (n, _) in enumerate(meta.host_lens) if i not in taken)), B - len(take)
+        rest = [x for i, x in enumerate(meta.host_lens) if i not in taken]
+        query_len, seqs, span = max(1, max(n for n, _ in rest)), len(rest), max(c for _, c in rest)
     mtiles = (query_len * G + 15) // 16
     if splits is None:
-        span = meta.max_seq_len or kv.page_size
         if sliding_window > 0:
             span = min(span, sliding_window + query_len)
-        splits = attn_splits(seqs, nkv, mtiles, span, sm_count(q.device), 3 if kv.dtype_name in ("q8", "q4") else 2)
+        splits = attn_plan.splits(seqs, nkv, mtiles, span, sm_count(q.device), 3 if kv.dtype_name in ("q8", "q4") else 2)
     ws_o = ws_ml = cnt = None
     if splits > 1 and B * nkv * mtiles > scratch(q.device).attn_counters.numel():
         splits = 1
