@@ -21,6 +21,7 @@ from ..models.config import ModelConfig
 from ..models.registry import act_dtype_for, config_from_checkpoint, load_checkpoint_weights
 from ..models.transformer import Transformer
 from ..models.weights import ModelWeights
+from ..ops import attn_plan
 from ..utils import profiler as _profiler
 from .kv_pool import BlockPool, KVCacheSpec, StateSlots, StateStore, make_block_pool
 from .runner import ModelRunner, StepResult
@@ -189,6 +190,7 @@ class LLM:
         free, total = torch.cuda.mem_get_info(self.device)
         budget = int(free - (1.0 - c.gpu_memory_utilization) * total)
         budget -= c.max_num_seqs * StateStore.slot_bytes(self.cfg.state_shapes, self.cfg.state_windows)
+        budget -= attn_plan.reserve_bytes(spec, c.max_model_len, c.max_num_seqs)
         fit = max(16, budget // max(spec.bytes_per_block() + extra_bytes_per_block, 1))
         return int(min(want, fit))
 

@@ -47,6 +47,16 @@ def pages_seen(rows: int, ctx: int, window: int) -> int:
     return (ctx + 15) // 16 - first_page(rows, ctx, window)
 
 
+def reserve_bytes(spec, max_len: int, max_seqs: int) -> int:
+    """What the converted pages of a layer can take in a step over a cache like ``spec`` (``KVCacheSpec``): memory that a server leaves
+    free beside its pool."""
+    if spec.dtype_name not in SOURCE_BYTES or spec.dtype_name == "bf16" or spec.page_size != 16:
+        return 0
+    layers = [spec.shape(i) for i in range(spec.n_layers)]
+    page = max((heads * 64 * width for heads, planes, width in layers if planes == 2 and width in (64, 128)), default=0)
+    return min(MAX_PAGES_BYTES, page * (-(-max_len // 16)) * max_seqs)
+
+
 def splits(seqs: int, nkv: int, mtiles: int, span: int, sms: int, per_sm: int) -> int:
     """CTA-level KV splits of the mma.sync kernel: as many as keep the grid within ONE wave of ``per_sm`` CTAs per SM (two, or three
     over quantized pages; a partly filled second wave doubles the kernel's time) while each warp of each split still sees a few

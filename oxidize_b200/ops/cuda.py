@@ -184,6 +184,7 @@ class Scratch:
         self.attn_o: Optional[torch.Tensor] = None
         self.attn_ml: Optional[torch.Tensor] = None
         self.attn_counters = self._new(65536, torch.int32, "attention split tickets", zero=True)
+        self.attn_pages: Optional[torch.Tensor] = None  # checked mode only
         self.dequant: Optional[torch.Tensor] = None
         self._cap_attn = None
         self._cap_dequant = None
@@ -213,6 +214,18 @@ class Scratch:
         if self.attn_ml is None or self.attn_ml.numel() < ml_floats:
             self.attn_ml = self._new(max(ml_floats, 1), torch.float32, "attention split-KV max / sum", old=self.attn_ml)
         return self.attn_o, self.attn_ml
+
+    def pages(self, n: int) -> Optional[torch.Tensor]:
+        """Room for n bf16 values of converted pages, for one call (its own, so that streams do not share it; in checked mode one
+        buffer between bands); None where the device has none left."""
+        try:
+            if self.guards is None or torch.cuda.is_current_stream_capturing():
+                return torch.empty(n, dtype=torch.bfloat16, device=self.device)
+            if self.attn_pages is None or self.attn_pages.numel() < n:
+                self.attn_pages = self._new(n, torch.bfloat16, "attention pages in bf16", old=self.attn_pages)
+            return self.attn_pages
+        except torch.OutOfMemoryError:
+            return None
 
     def dequant_buf(self, n: int) -> torch.Tensor:
         if torch.cuda.is_current_stream_capturing():
@@ -518,15 +531,18 @@ def _long_portions(q, kv, layer, meta, scale, window) -> List[int]:
     return known[1]
 
 
-def _paged_prefill(q, kv, layer, meta, take, scale, window, sink, out, out_scale, gate, gate_per_value) -> None:
+def _paged_prefill(q, kv, layer, meta, take, scale, window, sink, out, out_scale, gate, gate_per_value) -> bool:
+    """False, and nothing done, where there is no memory for converted pages."""
     T, nq, hd = q.shape
     nkv = kv.spec.heads(layer)
     take = sorted(take, key=lambda i: -meta.host_lens[i][1])  # the longest ways first
     rows, ctx = ([meta.host_lens[i][j] for i in take] for j in (0, 1))
     pages, cap = None, 0
     if kv.dtype_name != "bf16":
-        cap = sum((c + 15) // 16 for c in ctx)
-        pages = torch.empty(cap, nkv, 2, 16, hd, dtype=torch.bfloat16, device=q.device)
+        cap = sum(attn_plan.pages_seen(n, c, window) for n, c in zip(rows, ctx))
+        pages = scratch(q.device).pages(cap * nkv * 32 * hd)
+        if pages is None:
+            return False
     ints = ctypes.c_int * len(take)
     _check(lib().oxb_paged_prefill(q.data_ptr(), out.data_ptr(), kv.data[layer].data_ptr(), _p(kv.scales[layer]),
                                    meta.block_tables.data_ptr(), meta.seq_lens.data_ptr(), meta.query_start.data_ptr(), T,
@@ -534,6 +550,7 @@ def _paged_prefill(q, kv, layer, meta, take, scale, window, sink, out, out_scale
                                    len(take), window, scale, _p(sink), out.stride(0), out_scale, kv.num_blocks, _p(gate),
                                    0 if gate is None else gate.stride(0), int(gate_per_value), _p(pages), cap, _stream()),
            "oxb_paged_prefill")
+    return True
 
 
 def paged_attention(q, kv, layer, meta, scale, sliding_window=0, splits: Optional[int] = None, softcap: float = 0.0,
@@ -549,8 +566,7 @@ def paged_attention(q, kv, layer, meta, scale, sliding_window=0, splits: Optiona
         out = torch.empty_like(q)
     query_len, seqs, skip, span = max(1, meta.max_query_len), B, None, meta.max_seq_len or kv.page_size
     take = _long_portions(q, kv, layer, meta, scale, sliding_window) if splits is None and softcap == 0.0 else []
-    if take:
-        _paged_prefill(q, kv, layer, meta, take, scale, sliding_window, sink, out, out_scale, gate, gate_per_value)
+    if take and _paged_prefill(q, kv, layer, meta, take, scale, sliding_window, sink, out, out_scale, gate, gate_per_value):
         if len(take) == B:
             return out
         bits = 0

@@ -1,7 +1,9 @@
 """Rules that choose between kernels, on the CPU: they need only sizes."""
 import random
+from types import SimpleNamespace
 
 import pytest
+import torch
 
 from oxidize_b200.ops import attn_plan
 from oxidize_b200.ops import cuda as C
@@ -99,3 +101,23 @@ def test_converted_pages_stay_within_their_bytes():
 
 def test_more_sequences_than_the_mask_has_bits():
     assert _choose([(512, 512)] * (attn_plan.MAX_SEQS + 1), MANY) == []
+
+
+def test_a_server_leaves_room_for_converted_pages(monkeypatch):
+    from oxidize_b200.engine.kv_pool import KVCacheSpec
+    from oxidize_b200.engine.llm import LLM, EngineConfig
+
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda *_: (100 << 30, 180 << 30))
+    blocks = {}
+    for pages in ("bf16", "q8"):
+        spec = KVCacheSpec(80, 8, 128, 16, pages)
+        config = EngineConfig(max_model_len=131072, max_num_seqs=256, gpu_memory_utilization=0.99)
+        one = SimpleNamespace(config=config, device=torch.device("cuda"), cfg=SimpleNamespace(state_shapes=[], state_windows=[]))
+        blocks[pages] = LLM._auto_blocks(one, spec), spec.bytes_per_block()
+    free = int((100 - 0.01 * 180) * (1 << 30))
+    assert abs(blocks["bf16"][0] * blocks["bf16"][1] - free) < blocks["bf16"][1]
+    left = free - blocks["q8"][0] * blocks["q8"][1]
+    assert 0 <= left - attn_plan.MAX_PAGES_BYTES < blocks["q8"][1]
+    # no more than the longest sequences could take, and nothing for pages that are read as they are
+    assert attn_plan.reserve_bytes(KVCacheSpec(2, 2, 64, 16, "q4"), 100, 3) == 2 * 64 * 64 * 7 * 3
+    assert attn_plan.reserve_bytes(KVCacheSpec(2, 2, 64, 16, "bf16"), 100, 3) == attn_plan.reserve_bytes(KVCacheSpec(2, 2, 96, 16, "q4"), 100, 3) == 0

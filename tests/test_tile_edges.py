@@ -325,3 +325,36 @@ def test_long_portions_with_sinks_and_gates(C, monkeypatch, kvd, gates, sinks):
     if gates is not None:
         want = ref.head_gate(want, gate, SimpleNamespace(heads=8, width=128, gate=gates))
     assert _off(got, want) < (2.5e-3 if kvd == "bf16" else 6e-3)  # (as test_long_portions)
+
+
+@pytest.mark.parametrize("kvd", ["q8", "q4", "f16"])
+def test_long_portions_without_room_for_converted_pages(C, monkeypatch, kvd):
+    """An allocation that fails sends the step to the kernel that needs none."""
+    _take(monkeypatch, C, lambda i, n: n >= 32)
+    cpu, meta, gpu, on_gpu, q = _step(kvd, 128, 8, 2, LONG)
+    asked = []
+
+    def none_left(*size, **more):
+        if more.get("dtype") is torch.bfloat16:
+            asked.append(size)
+            raise torch.OutOfMemoryError("no room")
+        return torch.empty(*size, **more)
+
+    with monkeypatch.context() as m:
+        m.setattr(C, "torch", _Without(torch, empty=none_left))
+        m.setattr(C.scratch(torch.device("cuda")), "guards", None)
+        got = C.paged_attention(q.cuda(), gpu, 0, on_gpu, 128 ** -0.5, splits=None, out=torch.zeros_like(q.cuda()))
+    _check_status(C)
+    assert len(asked) == 1
+    assert _off(got, ref.paged_attention(q.float(), cpu, 0, meta, 128 ** -0.5)) < 6e-3  # (as test_long_portions)
+
+
+class _Without:
+    """A module with some of its names replaced."""
+
+    def __init__(self, module, **names):
+        self.__dict__.update(names)
+        self._module = module
+
+    def __getattr__(self, name):
+        return getattr(self._module, name)
