@@ -311,10 +311,6 @@ static __global__ void qk_rope_kvwrite_kernel(const __nv_bfloat16* __restrict__ 
   }
 }
 
-// The same for heads of 32 V values, a warp to a head and V neighbouring values to a lane: rotation partners are a shuffle away,
-// loads and stores are 2 V bytes wide and nothing goes through shared memory.  One value per thread and a CTA per head was
-// bound by its CTAs (24576 of them, 26 us, for 512 tokens x 48 heads of 128 into a q8 cache; four layers of a prefill of 512 take 65 us less
-// with this).  The one above stays for other widths and rotations.
 // N neighbouring floats on an N-float boundary
 template <int N>
 __device__ __forceinline__ void load_floats(const float* p, float* o) {
@@ -336,6 +332,10 @@ __device__ __forceinline__ void load_floats(const float* p, float* o) {
   }
 }
 
+// The same for heads of 32 V values, a warp to a head and V neighbouring values to a lane: rotation partners are a shuffle away,
+// loads and stores are 2 V bytes wide and nothing goes through shared memory.  512 tokens x 72 heads of 128: 16 us, where the
+// kernel above, bound by its CTAs, takes 48; one token, where the chain of loads is the time: 6.9 and 6.6.  The one above stays for
+// other widths and rotations.
 template <int V>
 static __global__ void __launch_bounds__(256)
 qk_rope_kvwrite_warp_kernel(const __nv_bfloat16* __restrict__ qkv, const int* __restrict__ positions, const int* __restrict__ slots,
@@ -395,26 +395,42 @@ qk_rope_kvwrite_warp_kernel(const __nv_bfloat16* __restrict__ qkv, const int* __
     }
     if (nw != nullptr) {
       load_floats<V>(nw + d0, w_n);
-      float ss = 0.f;
+      // the sum of squares in the order of the kernel above (32 neighbouring values pair by pair, furthest first, then those sums)
+      float t2[V];
 #pragma unroll
-      for (int j = 0; j < V; ++j) ss += v[j] * v[j];
-      const float r = rsqrtf(warp_sum(ss) / (float)HD + eps);
+      for (int j = 0; j < V; ++j) t2[j] = v[j] * v[j];
+#pragma unroll
+      for (int o = 16 / V; o > 0; o >>= 1) {
+#pragma unroll
+        for (int j = 0; j < V; ++j) t2[j] += __shfl_xor_sync(0xffffffffu, t2[j], o);
+      }
+#pragma unroll
+      for (int o = V / 2; o > 0; o >>= 1) {
+#pragma unroll
+        for (int j = 0; j < o; ++j) t2[j] += t2[j + o];
+      }
+      float ss = t2[0];
+#pragma unroll
+      for (int o = 16; o >= 32 / V; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      const float r = rsqrtf(ss / (float)HD + eps);
 #pragma unroll
       for (int j = 0; j < V; ++j) v[j] = v[j] * r * w_n[j];
     }
+    // v c + o s, rounded as the kernel above rounds it: the cache rows of both are the same bits
+    auto turn = [](float x, float c, float o, float sn) { return __fmaf_rn(x, c, __fmul_rn(o, sn)); };
     if (pairing == 0) {
       const int from = !turned ? lane : first ? lane + half / V : lane - half / V;
 #pragma unroll
       for (int j = 0; j < V; ++j) {
         const float o = __shfl_sync(0xffffffffu, v[j], from);
-        if (turned) v[j] = first ? (v[j] * c[j] - o * sn[j]) : (v[j] * c[j] + o * sn[j]);
+        if (turned) v[j] = turn(v[j], c[j], first ? -o : o, sn[j]);
       }
     } else if (turned) {
 #pragma unroll
       for (int j = 0; j < V; j += 2) {
         const float x = v[j], y = v[j + 1];
-        v[j] = x * c[j / 2] - y * sn[j / 2];
-        v[j + 1] = y * c[j / 2] + x * sn[j / 2];
+        v[j] = turn(x, c[j / 2], -y, sn[j / 2]);
+        v[j + 1] = turn(y, c[j / 2], x, sn[j / 2]);
       }
     }
   }
