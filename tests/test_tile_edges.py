@@ -358,3 +358,31 @@ class _Without:
 
     def __getattr__(self, name):
         return getattr(self._module, name)
+
+
+@pytest.mark.parametrize("kvd", ["bf16", "f32", "q8", "q4"])
+@pytest.mark.parametrize("hd,pairing,norm", [(64, "split_half", False), (64, "adjacent", True), (128, "split_half", True), (128, "adjacent", False),
+                                             (256, "split_half", True), (256, "adjacent", True)])
+def test_both_rotation_kernels_write_the_same_bits(C, kvd, hd, pairing, norm):
+    """Queries on an 8-byte boundary take the kernel of one value to a thread, the same on a 16-byte one a warp to a head."""
+    from types import SimpleNamespace
+
+    gen = torch.Generator().manual_seed(hd)
+    T, nq, nkv = 77, 5, 2
+    qkv = torch.randn(T, (nq + 2 * nkv) * hd, generator=gen).bfloat16()
+    norms = [(torch.rand(hd, generator=gen) + 0.5).cuda() if norm else None for _ in range(2)]
+    pos, slots = (torch.arange(T, dtype=torch.int32, device="cuda") * 31, torch.arange(T, dtype=torch.int32, device="cuda"))
+    rope = SimpleNamespace(inv_freq=ref.rope_inv_freq(hd, 10000.0, None, device="cuda"), pairing=pairing, mscale=1.0, n_heads=nq,
+                           n_kv_heads=nkv, head_dim=hd, max_pos=0)
+    seen = []
+    for offset in (0, 4):
+        room = torch.empty(qkv.numel() + 4, dtype=torch.bfloat16, device="cuda")
+        at = room[offset : offset + qkv.numel()].view(qkv.shape)
+        at.copy_(qkv)
+        kv = KVCache(KVCacheSpec(1, nkv, hd, 16, kvd), 8, torch.device("cuda"))
+        for d in kv.data + [s for s in kv.scales if s is not None]:
+            d.zero_()
+        q = C.qk_rope_kv_write(at, pos, slots, kv, 0, rope, *norms, 1e-6)
+        seen.append([q, kv.data[0]] + ([] if kv.scales[0] is None else [kv.scales[0]]))
+    _check_status(C)
+    assert all(torch.equal(a, b) for a, b in zip(*seen))
