@@ -360,6 +360,39 @@ class _Without:
         return getattr(self._module, name)
 
 
+@pytest.mark.parametrize("qtype,K", [("Q8_0", 512), ("Q8_0", 1536), ("Q8_0", 3584), ("Q6_K", 1024), ("Q6_K", 3072), ("Q6_K", 2048), ("Q4_K", 2048),
+                                     ("Q4_K", 6144)])
+@pytest.mark.parametrize("T,N", [(1, 1), (2, 33), (1, 4737), (2, 9473)])
+def test_packed_gemv_stream(C, qtype, K, T, N):
+    """Rows that end inside a segment, rings that wrap and that do not fill, rows that are no pairs or one for every warp and one more;
+    against the same activations in 8 bits, so that only sums and the output are rounded."""
+    gen = torch.Generator(device="cuda").manual_seed(N + K)
+    some = 257
+    w = qtensor_from_dense((torch.randn(some, K, generator=gen, device="cuda") * 0.05).cpu(), qtype, device="cuda")
+    dense = w.to("cpu").dense_cache().double().cuda()
+    again = -(-N // some)
+    w.data, w.shape, w._dense = w.data.repeat(again, 1)[:N].contiguous(), (N, K), None
+    x = torch.randn(T, K, generator=gen, device="cuda").bfloat16()
+    x[0, : K // 4] = 0
+    codes = x.float().view(T, -1, 32)
+    step = codes.abs().amax(-1, keepdim=True) / 127
+    codes = (torch.round(torch.where(step > 0, codes / step, 0)).double() * step.double()).view(T, K)
+    room = torch.full((T + 2, N + 3), 7.0, dtype=torch.bfloat16, device="cuda")
+    from oxidize_b200.ops import cuda_quant
+
+    C.configure(C.KernelOptions(gemv_wide=True))
+    try:
+        cuda_quant.linear_quant(x, w, room[1 : T + 1, 1 : N + 1], None, room.stride(0))
+    finally:
+        C.configure(C.KernelOptions())
+    _check_status(C)
+    got, want = room[1 : T + 1, 1 : N + 1].double(), (codes @ dense.t()).repeat(1, again)[:, :N]
+    # the output to bf16 (2^-9); a code of 8 bits may fall to the other side where a value lies between two (1 / 254 of 32 values' largest)
+    assert ((got - want).abs() <= want.abs() * 2 ** -8 + 0.01 * want.square().mean().sqrt()).all()
+    room[1 : T + 1, 1 : N + 1] = 7.0
+    assert (room == 7.0).all()
+
+
 @pytest.mark.parametrize("kvd", ["bf16", "f32", "q8", "q4"])
 @pytest.mark.parametrize("hd,pairing,norm", [(64, "split_half", False), (64, "adjacent", True), (128, "split_half", True), (128, "adjacent", False),
                                              (256, "split_half", True), (256, "adjacent", True)])
