@@ -228,11 +228,12 @@ __device__ __forceinline__ void attn_merge_rows(const AttnArgs& a, int G, int b,
 // and that of the output columns are free, so a lane takes whole words of codes: of a key's 32 channels under one scale, lane t4 takes
 // 8t4 .. 8t4 + 7, and the queries' fragments are put in the same order; of a value row's, lane g takes 4g .. 4g + 3, one for each of four
 // column tiles.  The sums of a key's channel groups are scaled apart, as are the probabilities for the values' groups.
-// (Decoding pages to bf16 rows in shared memory first took 1150 instructions a page and 139 KB, one CTA per SM: at 4 x 25000 q4 rows of
-// 8 heads, 128 wide, 273 us, now 65, of which the copies would take 20; 32 x 640 q8 rows 63 and 25.)
+// (4 x 25000 q4 rows of 8 heads, 128 wide: 65 us, of which the copies would take 20, where decoding pages to bf16 rows in shared memory
+// first, 1150 instructions a page and one CTA of 139 KB per SM, takes 273; 32 x 640 q8 rows 25 and 63.)
 // NR: halves of the 16-row tile that hold rows.  A decode step with at most 8 query heads to a key head fills one; the softmax, the
-// scaling of probabilities and half of the accumulators of the other are then left out (and with them 48 registers, which lets a
-// fourth CTA of the q4 form onto an SM).
+// scaling of probabilities and half of the accumulators of the other are then left out (4 x 25000 q4 rows 66.6 us, with whole tiles
+// 69.6; 32 x 640 q8 rows 27.6 and 28.8, launch included).  Three CTAs of the quantized forms fit an SM either way: at width 128 the
+// half tile takes the same 168 registers and spills 20 to 52 bytes beside them.
 template <int HD, int MODE, int NR>
 __global__ void __launch_bounds__(ATT_WARPS * 32, MODE == 0 ? 1 : 3)
 paged_attention_kernel(const AttnArgs a, int G /*q heads per kv head*/, const __grid_constant__ AttnSkip skip) {

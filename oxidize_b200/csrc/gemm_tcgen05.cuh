@@ -104,7 +104,7 @@ struct GemmStages {
   static constexpr bool A_IN_TMEM = QT != QT_BF16;
   // k-blocks per stage.  Packed weights: two.  The control warps' instructions are what a k-block costs there: a wait, a vote, a
   // fence, a commit and the addresses in between took the MMA warp 450 cycles next to the decoders, for 64 (16 tokens to a tile) to
-  // 256 (128 tokens) of tensor-core time; per pair of k-blocks they are paid once (Q4_K, 28672 x 4096, 32 tokens: 52 us before, 46 now).
+  // 256 (128 tokens) of tensor-core time; per pair of k-blocks they are paid once (Q4_K, 28672 x 4096, 32 tokens: 46 us, one by one 52).
   static constexpr int KPS = A_IN_TMEM ? 2 : 1;
   static constexpr int STAGE_BYTES = A_IN_TMEM ? KPS * GemmTile<TN>::B_BYTES : GemmTile<TN>::STAGE_BYTES;
   static constexpr int B_OFFSET = A_IN_TMEM ? 0 : GemmTile<TN>::A_BYTES;  // activation tile inside a stage
@@ -715,8 +715,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
   } else if (warp == GEMM_WARP_PACKED) {
     // ---------------- TMA producer of the packed super-blocks (tmW maps the packed rows as bytes): PRING boxes are in
     // flight or being decoded; a box is refilled as soon as every decoding warp has let go of it.  Weights are static, so
-    // none of this waits for the upstream kernel.  (A thread of the first decoding group used to do this: its group then came
-    // last with every super-block, and as the MMAs take k-blocks in order, everything waited for it.)
+    // none of this waits for the upstream kernel.  (Were it a decoding group's work, that group would come last with every
+    // super-block, and as the MMAs take k-blocks in order, everything would wait for it.)
     if constexpr (STAGED) if (qw.staged) {
       constexpr int SB = MmqStage<QT>::SB, PBYTES = MmqStage<QT>::BYTES;
       const bool leader = elect_one();
@@ -1129,7 +1129,7 @@ inline GemmPlan gemm_plan(int T, int N, int K, int splits_hint, int sm_count, in
   p.tn = T <= 16 ? 16 : T <= 32 ? 32 : T <= 64 ? 64 : T <= 128 ? 128 : 256;
   p.n_tiles = (N + GEMM_BM - 1) / GEMM_BM;
   if (packed && T > 128) {
-    // A k-block costs the decoders about as long as the products of 256 tokens take (550 and 512 cycles), so a tile of 256 tokens
+    // A k-block costs the decoders about as long as the products of 256 tokens take (520 and 512 cycles), so a tile of 256 tokens
     // takes little longer than one of 128 and decodes half as often: it is taken wherever it saves a wave.
     const int sms = sm_count > 0 ? sm_count : 148;
     const long long w256 = ((long long)p.n_tiles * groups * ((T + 255) / 256) + sms - 1) / sms;

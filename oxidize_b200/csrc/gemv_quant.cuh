@@ -362,9 +362,10 @@ gemv_quant_kernel(const uint8_t* __restrict__ W, size_t row_bytes, const __nv_bf
 
 // The same product as a stream: every warp owns a ring of segments of row pairs in shared memory that bulk copies fill, so how many
 // bytes are in flight does not depend on registers or on where a warp is in its arithmetic, and as the weights are static the
-// first rings (up to 105 KB per SM) are requested before the kernel waits for its activations.  One CTA of 16 warps per SM in
-// less than half of its shared memory: the next product's CTA fits beside it and has its rings filled when its turn comes.
-// 28672 x 4096, one token, launch included: Q4_K 28.7 us before, 24.6 now; Q6_K 49 and 39; Q8_0 57 and 41.
+// first rings (up to 105 KB per SM) are requested before the kernel waits for its activations.  One CTA of 16 warps per SM; while it
+// takes less than half of the shared memory (one token: rows of up to 32768 values in Q4_K, 6144 in Q6_K, 8192 in Q8_0; two: half of
+// that), the next product's CTA fits beside it and has its rings filled when its turn comes.
+// 28672 x 4096, one token, launch included, this kernel and gemv_quant_kernel: Q4_K 24.6 and 28.7 us; Q6_K 39 and 49; Q8_0 41 and 57.
 // gemv_quant_kernel stays for rows that are not whole warp iterations or not on 16-byte boundaries, and for more than two tokens.
 constexpr int GS_WARPS = 16, GS_ROWS = 2, GS_WARP_RING = 6720;
 template <int QT>
