@@ -6,11 +6,11 @@ other has a CTA for 16 rows and splits contexts.  So the choice goes by estimate
 knows of it, and names sequences: the tail of a long prompt can take one kernel and the prompt next to it the other.
 
 The constants are fits to one B200 (rows 32 to 2048 over contexts up to 32000; 8 to 64 query heads, groups of 1 to 8; windows;
-steps of up to 64 sequences), in microseconds; over 791 such steps what they choose is within 0.4 % of the better of all and none
-on average, 23 % at worst.  Around the line, at 8 query heads / 1 key head of 128 in bf16: 256 rows over 8000
-keys (8 CTAs) take 168 us here and 86 there, 512 rows 170 and 147, 1024 rows 172 and 279; 8 / 2 heads of 64: 1024 rows 172
-and 154, 2048 rows 174 and 266.  At 32 / 8 heads of 128: 64 rows over 8000 keys 168 and 86, 256 rows 174 and 272.  A portion of 500
-rows and a tail of 40 over 12000, 32 / 8 heads: 245 us both here, 242 both there, 103 apart.
+steps of up to 64 sequences), in microseconds; over 791 such steps what the estimates choose is within 0.4 % of the better of
+all and none on average, 23 % at worst.  Around the line, at 8 query heads / 1 key head of 128 in bf16: 256 rows over 8000 keys
+(8 CTAs) take 168 us here and 86 there, 512 rows 170 and 147, 1024 rows 172 and 279; 8 / 2 heads of 64: 1024 rows 172 and 154,
+2048 rows 174 and 266.  At 32 / 8 heads of 128: 64 rows over 8000 keys 168 and 86, 256 rows 174 and 272.  A portion of 500 rows and
+a tail of 40 over 12000, 32 / 8 heads: 245 us both here, 242 both there, 103 apart.
 """
 from __future__ import annotations
 
@@ -19,6 +19,11 @@ from typing import List, Sequence, Tuple
 
 MIN_ROWS = 32  # shorter portions are the other kernel's
 MAX_SEQS = 2048  # ... as are steps of more sequences (its mask of sequences has a bit for each)
+# Steps whose portions are all shorter than this are looked at only if their products alone, at 100 TFLOP/s, would take longer in the other
+# kernel: for long contexts, that is.  More of them would gain (32 prompts of 33 rows, 32 heads: 20 us here, 61 there), but prompts
+# of a hundred rows over q4 pages see little else than their own rows' codes, which the last bits of the layers before decide, and come out up
+# to 8 % apart between the kernels (either is up to 19 % from 64 bits).
+SHORT = 192
 MAX_PAGES_BYTES = 512 << 20  # converted pages of a layer, at most
 
 STEP, STEP_FIXED = 1.27, 6  # 64 keys of a CTA; what starting and ending a CTA costs, in such steps
@@ -81,6 +86,12 @@ def choose(lens: Sequence[Tuple[int, int]], nq: int, nkv: int, hd: int, pages: s
     def work(n, c):  # TFLOP x 1e6 of n rows, each over the keys it sees
         full = c - n / 2
         return 4e-6 * nq * hd * n * (min(full, window) if window > 0 else full)
+
+    if max(lens[i][0] for i in cand) < SHORT:
+        waves = -(-sum(-(-lens[i][0] * nq // 256) for i in cand) // sms)
+        walk = max(min(c, window + n) if window > 0 else c for n, c in (lens[i] for i in cand)) / 64
+        if 1.3 * waves * (walk + STEP_FIXED) + 6 > sum(work(*lens[i]) for i in cand) / 100 + 8:
+            return []
 
     # per sequence, for the tcgen05 kernel: work of its CTAs and of the longest (in steps), bytes of its pages, converted ones
     def alone(n, c):

@@ -61,7 +61,8 @@ FEW, SMALL, MANY = (8, 1, 128), (8, 2, 64), (32, 8, 128)
     ([(64, 8000)], MANY, "bf16", 0, []),  # 168 / 86
     ([(64, 8000)] * 4, MANY, "bf16", 0, [0, 1, 2, 3]),  # 172 / 276
     ([(256, 8000)], MANY, "bf16", 0, [0]),  # 174 / 272
-    ([(33, 33)] * 32, MANY, "bf16", 0, list(range(32))),  # 20 / 61
+    ([(33, 33)] * 32, MANY, "bf16", 0, []), ([(140, 140), (83, 83)], MANY, "q4", 0, []),  # short ones, over no long context
+    ([(161, 161), (146, 146), (122, 122)], (64, 8, 128), "q4", 0, [0, 1, 2]),
     ([(256, 8000)], FEW, "bf16", 1024, []),  # 33 / 27
     ([(256, 8000)], MANY, "bf16", 1024, [0]),  # 35 / 57
     ([(256, 8000)], FEW, "q8", 0, []),  # 169 / 119, conversion of the pages included
