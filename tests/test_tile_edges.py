@@ -419,3 +419,22 @@ def test_both_rotation_kernels_write_the_same_bits(C, kvd, hd, pairing, norm):
         seen.append([q, kv.data[0]] + ([] if kv.scales[0] is None else [kv.scales[0]]))
     _check_status(C)
     assert all(torch.equal(a, b) for a, b in zip(*seen))
+
+
+@pytest.mark.parametrize("kvd", ["bf16", "q8"])
+def test_long_portions_as_they_are_dispatched(C, kvd):
+    """A prompt that fills the SMs takes the tcgen05 kernel, the tail of a long one beside it does not; a step that is built anew on the
+    same object is looked at anew."""
+    lens = [(40, 12000), (500, 500)]
+    cpu, meta, gpu, on_gpu, q = _step(kvd, 128, 32, 8, lens)
+    q = q.cuda()
+    assert C._long_portions(q, gpu, 0, on_gpu, 0.09, 0) == [1]
+    got = C.paged_attention(q, gpu, 0, on_gpu, 0.09)
+    _check_status(C)
+    want = ref.paged_attention(q.float().cpu(), cpu, 0, meta, 0.09)
+    assert _off(got, want) < (2.5e-3 if kvd == "bf16" else 6e-3)  # (as test_long_portions)
+    assert C._long_portions(q, gpu, 0, on_gpu, 0.09, 0) == [1]
+    on_gpu.host_lens = [(600, 700), (5, 60)]
+    assert C._long_portions(q, gpu, 0, on_gpu, 0.09, 0) == [0]
+    on_gpu.host_lens = None
+    assert C._long_portions(q, gpu, 0, on_gpu, 0.09, 0) == []
